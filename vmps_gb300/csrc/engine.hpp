@@ -156,9 +156,9 @@ struct GSeg  { int64_t b_off; int32_t term_begin, term_count; int32_t lda, ldb, 
 struct GTile { int64_t c_off; int32_t ldc, row0, col0, tm, tn, seg_begin, seg_end, step0, nsteps, rstride, nrhs; };
 // at most this many A terms per segment (the FP64 kernel stages them in shared memory)
 constexpr int kMaxTerms = 16;
-// FP64 engine tiles are at most 64 x 64 (rows split on multiples of 16, columns
-// on multiples of 8); tcgen05 engine tiles at most 128 x 256
-constexpr int kTileMax = 64;
+// FP64 engine tiles are at most 16 x 16; tcgen05 engine tiles at most 128 x 256
+// (rows split on multiples of 16)
+constexpr int kTileMax = 16;
 constexpr int kUmmaTileM = 128, kUmmaTileN = 256;
 constexpr int kUmmaBK = 32;   // K extent of one tcgen05 engine step
 
@@ -258,7 +258,7 @@ struct SplitTiling {
 };
 // FP64 plan: two phases, the second sums first-stage products on the fly
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z,
-               const DevLayout& O, bool transX, bool transZ, int tile_m, int tile_n);
+               const DevLayout& O, bool transX, bool transZ);
 // Split-precision plan for the tcgen05 engine: op(X), Y and the chain-scaled
 // copies c*op(Z) in panels; phase 1 computes the intermediates T = op(X)Y into
 // panels, phase 2 the outputs as K-concatenations over chains.

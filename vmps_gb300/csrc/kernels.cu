@@ -1,8 +1,8 @@
 // CUDA kernels of the GB300 effective-Hamiltonian engine (sm_103a).
 //
-// gg_fp64  : grouped GEMM, FP64 operands, DMMA (mma.sync m8n8k4 f64) -- the
-//            plain drop-in form, bit-for-bit the same arithmetic type as the
-//            Eigen path of pivot/DmrgPivotMatrix1.h:236-262.
+// gg_fp64  : grouped GEMM, FP64 operands, FP64 FMAs -- the plain drop-in form,
+//            the arithmetic type of the Eigen path of
+//            pivot/DmrgPivotMatrix1.h:236-262.
 // The split-precision (BF16x3) grouped GEMM is the tcgen05 engine in
 // umma.cu; this file holds its operand preparation (FP64 -> bf16 hi/lo
 // panels) and the vector kernels.
@@ -23,168 +23,119 @@
 
 namespace vmps {
 
-// ---------------------------------------------------------------------------
-// Operand staging of the FP64 engine.  Device blocks are column-major with ld a
-// multiple of 8, start offsets aligned to 32 elements and zero padding, and tile
-// origins are multiples of 16 (rows) / 8 (columns), so every 2-element (16-byte)
-// group read below is aligned and stays inside its block's padded storage.  Groups whose
-// first element lies outside the tile are replaced by zeros; elements past the
-// block edge inside a group are either zero padding or rows/columns that only
-// reach output entries the epilogue masks off.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void ldg2(const double* p, double (&v)[2]) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-    v[0] = a.x; v[1] = a.y;
-}
-
 // ===========================================================================
-// FP64 grouped GEMM: tile <= 64x64, 128 threads (2x2 warps of 32x32), BK = 16,
-// DMMA m8n8k4.  Shared layouts follow the contiguous global dimension:
-//   A row-contiguous  -> As[k][m] (stride 68)   A k-contiguous -> As[m][k] (stride 20)
-//   B k-contiguous    -> Bs[n][k] (stride 20)   B col-contiguous -> Bs[k][n] (stride 68)
-// (strides keep every half-warp of fragment reads on distinct banks).
+// FP64 grouped GEMM: tiles of at most 16 x 16, 128 threads, one output element
+// per thread and pass, scalar FMAs.
+//
+// GB300's FP64 pipe retires half an FMA per clock and SM quadrant whichever
+// instruction feeds it (an 8x8x4 DMMA holds its quadrant for 512 clocks), so DMMA
+// has no rate to gain and loses what its fragments round up: the blocks of these
+// tensors are 5 to 200 wide.  64 x 64 DMMA tiles left an 11 x 11 block to one
+// warp of one SM (72 us per launch at D = 64, now ~15); here the elements of a
+// tile spread over all four quadrants without rounding, and the tiles over more
+// SMs.  Large blocks gain as well: whole D = 1024 and 4096 two-site HxVs went from
+// 0.76 to 0.43 ms and from 17.9 to 16.3 ms, the FP64 pipe bounding both.  Small
+// ones are bound by the latency of the segment chain, so the segments and terms
+// of a tile come to shared memory first and each K chunk's loads are issued one
+// chunk ahead.
 // ===========================================================================
 namespace f64k {
-constexpr int BM = 64, BN = 64, BK = 16, NT = 128;
-constexpr int SMN = 68;   // [k][m] / [k][n] row stride (doubles)
-constexpr int SKK = 20;   // [m][k] / [n][k] row stride (doubles)
-constexpr int OP_ELEMS = BM * SKK > BK * SMN ? BM * SKK : BK * SMN;   // 1280 vs 1088
+constexpr int T = kTileMax, NT = 128, BK = 16, LD = T + 1;
+constexpr int SEGS = 32;                 // segments (and their terms) staged at a time
+constexpr int PER = T * BK / NT;         // operand elements a thread stages per chunk
 }
 
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
-__global__ void __launch_bounds__(f64k::NT, 3) gg_fp64_kernel(GGArgs g) {
+__global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
     using namespace f64k;
-    __shared__ __align__(16) double As[2][OP_ELEMS];
-    __shared__ __align__(16) double Bs[2][OP_ELEMS];
+    __shared__ double As[2][BK * LD], Bs[2][BK * LD];   // [k][row], [k][column]
+    __shared__ GSeg sseg[SEGS];
+    __shared__ GTerm sterm[SEGS * kMaxTerms];
     const GTile tile = g.tiles[blockIdx.x];
     const double* __restrict__ A = (const double*)g.A;
     const double* __restrict__ B = (const double*)g.B;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    const int mrem = tile.tm, nrem = tile.tn;
+    const int tid = threadIdx.x, tm = tile.tm, tn = tile.tn, ne = tm * tn;
     const bool tA = g.transA, tB = g.transB;
+    // the output elements of this thread, column by column; a second one for tiles of more than 128
+    const int e1 = tid + NT;
+    const bool on0 = tid < ne, on1 = e1 < ne;
+    const int j0 = on0 ? tid / tm : 0, i0 = on0 ? tid - j0 * tm : 0;
+    const int j1 = on1 ? e1 / tm : 0, i1 = on1 ? e1 - j1 * tm : 0;
+    double acc0 = 0.0, acc1 = 0.0;
 
-    double acc[4][4][2];
+    for (int sb = tile.seg_begin; sb < tile.seg_end; sb += SEGS) {
+        const int ns = min(SEGS, tile.seg_end - sb);
+        __syncthreads();   // the staged lists and both chunk buffers are free
+        for (int s = tid; s < ns; s += NT) sseg[s] = g.segs[sb + s];
+        __syncthreads();
+        const int tb = sseg[0].term_begin, nt = sseg[ns - 1].term_begin + sseg[ns - 1].term_count - tb;
+        for (int t = tid; t < nt; t += NT) sterm[t] = g.terms[tb + t];
+        __syncthreads();
+        double ra[PER], rb[PER];
+        auto stage = [&](int s, int k0) {
+            const GSeg& sg = sseg[s];
+            const int krem = sg.K - k0, t0 = sg.term_begin - tb;
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
-    // each thread stages 4 double2 of A and 4 of B per BK step
-    double ra[4][2], rb[4][2];
-    auto stage = [&](int s, int k0) {
-        const GSeg sg = g.segs[s];
-        const int krem = sg.K - k0;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int v = tid + NT * r;   // 512 pairs per operand tile
-            int i, k;
-            if (!tA) { i = (v & 31) * 2; k = v >> 5; }      // m-pairs along rows, 16 k columns
-            else     { k = (v & 7) * 2;  i = v >> 3; }      // k-pairs, 64 rows
-            ra[r][0] = ra[r][1] = 0.0;
-            if (i < mrem && k < krem) {
-                const int64_t e = tA ? ((int64_t)(k0 + k) + (int64_t)(tile.row0 + i) * sg.lda)
-                                     : ((int64_t)(tile.row0 + i) + (int64_t)(k0 + k) * sg.lda);
-                for (int t = 0; t < sg.term_count; ++t) {
-                    const GTerm tm = g.terms[sg.term_begin + t];
-                    double x[2];
-                    ldg2(A + tm.off + e, x);
-                    ra[r][0] = fma(tm.coef, x[0], ra[r][0]);
-                    ra[r][1] = fma(tm.coef, x[1], ra[r][1]);
+            for (int r = 0; r < PER; ++r) {
+                const int v = tid + NT * r, lo = v & (T - 1), hi = v / T;
+                const int i = tA ? hi : lo, k = tA ? lo : hi;   // lanes run along the contiguous dimension
+                ra[r] = 0.0;
+                if (i < tm && k < krem) {
+                    const int64_t e = tA ? (int64_t)(k0 + k) + (int64_t)(tile.row0 + i) * sg.lda
+                                         : (int64_t)(tile.row0 + i) + (int64_t)(k0 + k) * sg.lda;
+                    for (int t = 0; t < sg.term_count; ++t) {
+                        const GTerm tm_ = sterm[t0 + t];
+                        ra[r] = fma(tm_.coef, __ldg(A + tm_.off + e), ra[r]);
+                    }
+                }
+                const int j = tB ? lo : hi, kb = tB ? hi : lo;
+                rb[r] = 0.0;
+                if (j < tn && kb < krem) {
+                    const int64_t e = tB ? (int64_t)(tile.col0 + j) + (int64_t)(k0 + kb) * sg.ldb
+                                         : (int64_t)(k0 + kb) + (int64_t)(tile.col0 + j) * sg.ldb;
+                    rb[r] = __ldg(B + sg.b_off + e);
                 }
             }
-            int j, kb;
-            if (!tB) { kb = (v & 7) * 2;  j = v >> 3; }
-            else     { j = (v & 31) * 2;  kb = v >> 5; }
-            rb[r][0] = rb[r][1] = 0.0;
-            if (j < nrem && kb < krem) {
-                const int64_t e = tB ? ((int64_t)(tile.col0 + j) + (int64_t)(k0 + kb) * sg.ldb)
-                                     : ((int64_t)(k0 + kb) + (int64_t)(tile.col0 + j) * sg.ldb);
-                ldg2(B + sg.b_off + e, rb[r]);
-            }
-        }
-    };
-    auto commit = [&](int buf) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int v = tid + NT * r;
-            if (!tA) { const int i = (v & 31) * 2, k = v >> 5;
-                       *reinterpret_cast<double2*>(&As[buf][k * SMN + i]) = make_double2(ra[r][0], ra[r][1]); }
-            else     { const int k = (v & 7) * 2, i = v >> 3;
-                       *reinterpret_cast<double2*>(&As[buf][i * SKK + k]) = make_double2(ra[r][0], ra[r][1]); }
-            if (!tB) { const int kb = (v & 7) * 2, j = v >> 3;
-                       *reinterpret_cast<double2*>(&Bs[buf][j * SKK + kb]) = make_double2(rb[r][0], rb[r][1]); }
-            else     { const int j = (v & 31) * 2, kb = v >> 5;
-                       *reinterpret_cast<double2*>(&Bs[buf][kb * SMN + j]) = make_double2(rb[r][0], rb[r][1]); }
-        }
-    };
-
-    int seg = tile.seg_begin, k0 = 0;
-    // DMMA work is skipped, warp-uniformly, for 8x8 fragments wholly outside the
-    // tile and for k-quads past the end of the segment: GB300's FP64 MMA rate is
-    // fixed, so MMAs on zero padding of small blocks cost full time
-    const int mi_live = mrem > wm ? min(4, (mrem - wm + 7) >> 3) : 0;
-    const int ni_live = nrem > wn ? min(4, (nrem - wn + 7) >> 3) : 0;
-    const bool warp_live = mi_live > 0 && ni_live > 0;
-    if (seg < tile.seg_end) {
-        stage(seg, k0);
-        int buf = 0;
+        };
+        int s = 0, k0 = 0, buf = 0;
+        stage(0, 0);
         while (true) {
-            commit(buf);
+#pragma unroll
+            for (int r = 0; r < PER; ++r) {
+                const int v = tid + NT * r, lo = v & (T - 1), hi = v / T;
+                As[buf][tA ? lo * LD + hi : hi * LD + lo] = ra[r];
+                Bs[buf][tB ? hi * LD + lo : lo * LD + hi] = rb[r];
+            }
             __syncthreads();
-            const int kcur = min(BK, g.segs[seg].K - k0);   // valid k of the step in `buf`
-            int ns = seg, nk = k0 + BK;
-            if (nk >= g.segs[seg].K) { nk = 0; ++ns; }
-            const bool more = ns < tile.seg_end;
-            if (more) stage(ns, nk);
-            if (warp_live) {
-                const int g4 = lane >> 2, t4 = lane & 3;
-#pragma unroll
-                for (int kq = 0; kq < BK; kq += 4) {
-                    if (kq >= kcur) break;
-                    double af[4], bf[4];
-#pragma unroll
-                    for (int mi = 0; mi < 4; ++mi) {
-                        const int m = wm + mi * 8 + g4, k = kq + t4;
-                        af[mi] = tA ? As[buf][m * SKK + k] : As[buf][k * SMN + m];
+            const int kc = min(BK, sseg[s].K - k0);
+            k0 += BK;
+            if (k0 >= sseg[s].K) { k0 = 0; ++s; }
+            const bool more = s < ns;
+            if (more) stage(s, k0);
+            if (on0) {
+                const double* a = As[buf];
+                const double* b = Bs[buf];
+                if (on1) {
+#pragma unroll 4
+                    for (int k = 0; k < kc; ++k) {
+                        acc0 = fma(a[k * LD + i0], b[k * LD + j0], acc0);
+                        acc1 = fma(a[k * LD + i1], b[k * LD + j1], acc1);
                     }
-#pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) {
-                        const int n = wn + ni * 8 + g4, k = kq + t4;
-                        bf[ni] = tB ? Bs[buf][k * SMN + n] : Bs[buf][n * SKK + k];
-                    }
-#pragma unroll
-                    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                        for (int ni = 0; ni < 4; ++ni)
-                            if (mi < mi_live && ni < ni_live) dmma(acc[mi][ni][0], acc[mi][ni][1], af[mi], bf[ni]);
+                } else {
+#pragma unroll 4
+                    for (int k = 0; k < kc; ++k) acc0 = fma(a[k * LD + i0], b[k * LD + j0], acc0);
                 }
             }
             if (!more) break;
-            seg = ns; k0 = nk;
             buf ^= 1;
         }
     }
-    double* __restrict__ C = (double*)g.C;
-    const int g4 = lane >> 2, t4 = lane & 3;
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int r = wm + mi * 8 + g4, c = wn + ni * 8 + t4 * 2 + h;
-                if (r < mrem && c < nrem) {
-                    const int64_t gr = tile.row0 + r, gc = tile.col0 + c;
-                    const int64_t e = g.transC ? (gc + gr * tile.ldc) : (gr + gc * tile.ldc);
-                    C[tile.c_off + e] = acc[mi][ni][h];
-                }
-            }
+    double* __restrict__ C = (double*)g.C + tile.c_off;
+    auto put = [&](int i, int j, double x) {
+        const int64_t gr = tile.row0 + i, gc = tile.col0 + j;
+        C[g.transC ? gc + gr * tile.ldc : gr + gc * tile.ldc] = x;
+    };
+    if (on0) put(i0, j0, acc0);
+    if (on1) put(i1, j1, acc1);
 }
 
 // ---------------------------------------------------------------------------

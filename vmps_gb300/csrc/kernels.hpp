@@ -39,7 +39,7 @@ struct PanelPiece { int64_t src_off, dst_off; int32_t rows, cols, src_ld, dst_pi
 struct PackBlock { int64_t coff, doff, rows, cols, ld; double scale; };
 
 cudaError_t kernels_init();
-// FP64 grouped GEMM (DMMA)
+// FP64 grouped GEMM
 cudaError_t launch_gg64(const GGArgs& a, cudaStream_t st);
 // split-precision (BF16x3) grouped GEMM, tcgen05 engine (umma.cu): persistent,
 // TMA-fed, tiles up to 128 x 256; out_split = 1: C is a bf16 [hi|lo] panel arena,

@@ -740,7 +740,7 @@ static DevPlan& get_plan(vmps_pivot* p, int prec) {
         throw std::invalid_argument("unknown precision");
     DevPlan& dp = p->plans[prec];
     if (dp.ready) return dp;
-    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, 64, 64);
+    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false);
     else if (prec == VMPS_PREC_TF32X3) {
         dp.plan = make_split_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, 1, SplitTiling(), true);
         schedule_and_validate(dp.plan, p->ctx->num_sms);
@@ -2652,7 +2652,7 @@ static DevPlan& env_plan(vmps_env* e, int prec) {
     // left: X = Abra^dagger, Y = Eold, Z = Aket;  right: X = Aket, Y = Eold, Z = Abra^dagger
     const DevLayout& X = L ? e->Bd : e->Kd;
     const DevLayout& Z = L ? e->Kd : e->Bd;
-    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L, 64, 64);
+    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
     else {
         dp.plan = make_split_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
         schedule_and_validate(dp.plan, e->ctx->num_sms);

@@ -771,8 +771,8 @@ static std::vector<std::pair<int64_t, int64_t>> split_extent(int64_t m, int64_t 
 
 // append tiles of an m x n output block whose segments are [sb, se)
 void add_tiles(PhasePlan& ph, int64_t c_off, int64_t ldc, int64_t m, int64_t n, int32_t sb, int32_t se, int tile_m,
-               int tile_n, int col_gran = 8) {
-    for (const auto& rs : split_extent(m, 16, tile_m))
+               int tile_n, int col_gran = 8, int row_gran = 16) {
+    for (const auto& rs : split_extent(m, row_gran, tile_m))
         for (const auto& cs : split_extent(n, col_gran, tile_n)) {
             GTile t{};
             t.c_off = c_off;
@@ -948,14 +948,14 @@ PhasePlan make_product_plan(const DevLayout& A, const DevLayout& B, const DevLay
             ph.segs.push_back(s);
             ph.flops += 2.0 * A.rows[i] * A.cols[i] * B.cols[j];
         }
-        add_tiles(ph, C.off[k], C.ld[k], C.rows[k], C.cols[k], sb, (int32_t)ph.segs.size(), kTileMax, kTileMax);
+        add_tiles(ph, C.off[k], C.ld[k], C.rows[k], C.cols[k], sb, (int32_t)ph.segs.size(), kTileMax, kTileMax, 1, 1);
     }
     sort_tiles(ph);
     return ph;
 }
 
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z, const DevLayout& O,
-               bool transX, bool transZ, int tile_m, int tile_n) {
+               bool transX, bool transZ) {
     Plan P;
     // shapes: op(X) m x k, Y k x n, op(Z) n x p, out m x p
     auto xm = [&](int64_t x) { return transX ? X.cols[x] : X.rows[x]; };
@@ -1017,6 +1017,10 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
     }
     P.association = (f_yz < f_xy) ? 1 : 0;
 
+    auto tiles_of = [&](PhasePlan& ph, int64_t c_off, int64_t ldc, int64_t m, int64_t n, int32_t sb, int32_t se) {
+        add_tiles(ph, c_off, ldc, m, n, sb, se, kTileMax, kTileMax, 1, 1);
+    };
+
     // ---- intermediates
     std::unordered_map<Key4, int64_t, Key4Hash> idict;
     std::vector<std::pair<int64_t, int64_t>> ipairs;   // (x,y) or (y,z)
@@ -1069,7 +1073,7 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         int32_t sb = (int32_t)p1.segs.size();
         p1.segs.push_back(s);
         p1.flops += 2.0 * trows[j] * tcols[j] * K;
-        add_tiles(p1, P.T.off[j], P.T.ld[j], trows[j], tcols[j], sb, sb + 1, tile_m, tile_n);
+        tiles_of(p1, P.T.off[j], P.T.ld[j], trows[j], tcols[j], sb, sb + 1);
     }
     sort_tiles(p1);
 
@@ -1143,8 +1147,8 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         for (int32_t s = sb; s < se; ++s) { kk += p2.segs[s].K; kt += (double)p2.segs[s].K * p2.segs[s].term_count; }
         p2.flops += 2.0 * m * p * kk;
         P.flops_p2_unsummed += 2.0 * m * p * kt;
-        if (P.association == 0) add_tiles(p2, O.off[o], O.ld[o], m, p, sb, se, tile_m, tile_n);
-        else add_tiles(p2, O.off[o], O.ld[o], p, m, sb, se, tile_m, tile_n);
+        if (P.association == 0) tiles_of(p2, O.off[o], O.ld[o], m, p, sb, se);
+        else tiles_of(p2, O.off[o], O.ld[o], p, m, sb, se);
         i = j;
     }
     // output blocks that receive no product are still written (with zeros), as the
@@ -1155,8 +1159,8 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         const int32_t sb = (int32_t)p2.segs.size();
         for (size_t o = 0; o < O.rows.size(); ++o)
             if (!seen[o]) {
-                if (P.association == 0) add_tiles(p2, O.off[o], O.ld[o], O.rows[o], O.cols[o], sb, sb, tile_m, tile_n);
-                else add_tiles(p2, O.off[o], O.ld[o], O.cols[o], O.rows[o], sb, sb, tile_m, tile_n);
+                if (P.association == 0) tiles_of(p2, O.off[o], O.ld[o], O.rows[o], O.cols[o], sb, sb);
+                else tiles_of(p2, O.off[o], O.ld[o], O.cols[o], O.rows[o], sb, sb);
             }
     }
     sort_tiles(p2);
