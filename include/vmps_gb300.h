@@ -46,7 +46,11 @@ extern "C" {
 #define VMPS_E_UNSUPPORTED  -7
 
 /* ---- arithmetic of the block products --------------------------------------*/
-#define VMPS_PREC_FP64       0   /* plain FP64 (DMMA), parity with the Eigen path */
+#define VMPS_PREC_FP64       0   /* FP64, parity with the Eigen path: FP64 FMAs, or for large plans
+                                    the tensor cores on an error-free splitting of the operands, whose
+                                    error is no larger (a row or column with an Inf or NaN gives NaN);
+                                    the environment variable VMPS_FP64_ENGINE = auto | fma | slices
+                                    pins the choice                                            */
 #define VMPS_PREC_BF16X3     1   /* hi*hi + hi*lo + lo*hi bf16 products, FP32 accumulate */
 #define VMPS_PREC_TF32X3     2   /* the same three products with TF32 hi/lo operands (3xTF32): about
                                     2^-21 relative per product against 2^-16, at half the bf16 tensor

@@ -211,6 +211,51 @@ struct PhasePlan {
     double flops = 0;
 };
 
+// ---------------------------------------------------------------------------
+// FP64 plans on the tensor cores (slices.cu): operands as panels of seven base-512
+// digit slices in bf16 with one exponent per panel row.  Element (row i, K index k)
+// of slice s is at off + i*pitch + (k/32)*224 + s*32 + k%32, pitch = 7*kpad.
+// ---------------------------------------------------------------------------
+constexpr int kSlices = 7;
+constexpr int kSliceTileM = 128, kSliceTileN = 32;
+constexpr int kSliceK = 32;          // K extent of one step
+constexpr int kSliceFlushK = 64;     // K columns an FP32 accumulator sums exactly
+constexpr int kSliceSumK = 192;      // K columns whose flushes a 64-bit integer sums exactly
+constexpr int kSliceBad = 1 << 20;   // exponent of a row that holds an Inf or NaN
+// one block to slice: panel row i is source row i (trans 1) or source column i (trans 0)
+// of the sum of the terms' blocks (same leading dimension)
+struct SliceBlock { int64_t dst_off; int32_t erow, rows, K, pitch, trans, ld, term_begin, term_count; };
+struct SlicePiece { int32_t block, row0; };   // 32 panel rows of a block
+struct SliceOperand {
+    PanelArena arena;
+    std::vector<OpBlock> op;          // off, outer (rows), K, cls, row, pitch; pad = first exponent row
+    std::vector<SliceBlock> blocks;
+    std::vector<GTerm> terms;
+    std::vector<SlicePiece> pieces;
+    int64_t rows = 0;                 // exponents
+};
+// one K step: descriptors, slice coordinates (7 * K / 32) and panel rows of the A and B boxes
+struct SliceStep { int32_t amap, bmap, az, bz, ay, by, arows, flags; };
+constexpr int kSliceHalf = 1, kSliceFirst = 2, kSliceLast = 4, kSliceNarrow = 8;   // one K16 slice; group ends; tn <= 16
+// one flush: exponents of the tile's first row and column; kSliceSumEnd: the open sum of flushes
+// (equal exponents, at most kSliceSumK columns) ends with this one
+struct SliceGroup { int32_t ea, eb, flags, pad; };
+constexpr int kSliceSumEnd = 1;
+struct SliceTile { int64_t c_off; int32_t ldc, row0, col0, tm, tn, step0, nsteps, group0, ngroups, pad; };
+struct SliceSeg { int32_t a, b; };       // operand blocks (indices into SliceOperand::op), K of the A block
+struct SlicePhase {
+    std::vector<SliceSeg> segs;
+    std::vector<std::array<int32_t, 2>> tile_segs;   // segment range of each tile
+    std::vector<SliceTile> tiles;
+    std::vector<SliceStep> steps;
+    std::vector<SliceGroup> groups;
+    std::vector<MapKey> amaps, bmaps;
+    std::vector<int32_t> cta_tiles;
+    int ncta = 0;
+    int32_t max_arows = 16;
+    bool one_sum = true, one_flush = true;   // every tile is one segment of K <= kSliceSumK; of K <= kSliceFlushK
+};
+
 enum Slot { SLOT_X = 0, SLOT_Y = 1, SLOT_Z = 2, SLOT_OUT = 3, SLOT_T = 4 };
 
 // Split-precision operand preparation: one block of a column-major FP64 source
@@ -248,6 +293,10 @@ struct Plan {
     // Offsets, pitches and TMA x coordinates are in elements either way (x = 2 * k0).
     int elt = 2;
     int kstep = kUmmaBK;
+    // FP64 plans on the tensor cores: X, Y, Z and the summed first-stage products S
+    bool slices = false;
+    SliceOperand sx, sy, sz, ss;
+    SlicePhase s1, s2;
 };
 // Tile options of a split-precision plan (chosen by the autotuner): the N caps of
 // the phase-1 and phase-2 tiles (multiples of 32, at most kUmmaTileN) and the
@@ -256,9 +305,10 @@ struct SplitTiling {
     int ncap1 = 256, ncap2 = 256, splitk = 1;
     bool operator==(const SplitTiling& o) const { return ncap1 == o.ncap1 && ncap2 == o.ncap2 && splitk == o.splitk; }
 };
-// FP64 plan: two phases, the second sums first-stage products on the fly
+// FP64 plan: two phases, the second sums first-stage products on the fly; once: applied a single
+// time, so that the slices of X and Z are made for it alone
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z,
-               const DevLayout& O, bool transX, bool transZ);
+               const DevLayout& O, bool transX, bool transZ, bool once = false);
 // Split-precision plan for the tcgen05 engine: op(X), Y and the chain-scaled
 // copies c*op(Z) in panels; phase 1 computes the intermediates T = op(X)Y into
 // panels, phase 2 the outputs as K-concatenations over chains.
@@ -279,6 +329,9 @@ PhasePlan make_product_plan(const DevLayout& A, const DevLayout& B, const DevLay
 // longest-first to the least-loaded CTA and stored CTA by CTA.
 void schedule_tma(PhasePlan& ph, int ncta, const std::vector<OpBlock>& A, const std::vector<OpBlock>& B,
                   int kstep = kUmmaBK);
+// The same for the FP64 slice engine, and its invariants (throws std::logic_error)
+void schedule_slices(SlicePhase& ph, int ncta, const SliceOperand& A, const SliceOperand& B);
+void validate_slices(const SlicePhase& ph, const SliceOperand& A, const SliceOperand& B);
 // TMA box heights, the smallest that covers the tile: fine = the tile's rows
 // (columns) rounded up to 16; coarse (fewer descriptors) = A boxes of 16/32/64/128
 // rows, B boxes a multiple of 32 up to 256 (16 for the narrowest)

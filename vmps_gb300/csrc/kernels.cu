@@ -2,7 +2,8 @@
 //
 // gg_fp64  : grouped GEMM, FP64 operands, FP64 FMAs -- the plain drop-in form,
 //            the arithmetic type of the Eigen path of
-//            pivot/DmrgPivotMatrix1.h:236-262.
+//            pivot/DmrgPivotMatrix1.h:236-262; large FP64 plans run on the
+//            tensor cores (slices.cu) instead.
 // The split-precision (BF16x3) grouped GEMM is the tcgen05 engine in
 // umma.cu; this file holds its operand preparation (FP64 -> bf16 hi/lo
 // panels) and the vector kernels.
@@ -531,6 +532,7 @@ static int grid_for(int64_t n, int threads, int cap) {
 // before any launch or stream capture)
 cudaError_t kernels_init() {
     cudaError_t e = umma_init();
+    if (e == cudaSuccess) e = slices_init();
     return e != cudaSuccess ? e : lz_init();
 }
 

@@ -58,6 +58,36 @@ cudaError_t launch_panel_split_f32(const PanelPiece* pieces, int np, const float
 cudaError_t launch_prep_tf32(const PrepBlock* pb, int nb, const double* src, void* dst, cudaStream_t st);
 cudaError_t launch_panel_split_tf32(const PanelPiece* pieces, int np, const double* src, const float* srcf, void* dst,
                                     cudaStream_t st);
+// FP64 on the tensor cores (slices.cu): operand slices, and the grouped GEMM on them
+struct SliceArgs {
+    const SlicePiece* pieces;
+    const SliceBlock* blocks;
+    const GTerm* terms;
+    const double* src;
+    void* dst;        // digit panels
+    int32_t* exps;    // row exponents
+    int npieces;
+    int kcache;       // K indices of 32 rows kept in shared memory: a multiple of 32 up to kSliceCacheK
+};
+constexpr int kSliceCacheK = 256;
+struct SliceGemmArgs {
+    const SliceTile* tiles;
+    const SliceStep* steps;
+    const SliceGroup* groups;
+    const int32_t* cta_tiles;
+    const int32_t* ea;   // row exponents of A and B (readable kSliceTileM past the last)
+    const int32_t* eb;
+    double* C;
+    int* err;
+    int ncta;
+    int max_arows;       // rows of the phase's largest A box
+    int one_sum, one_flush;   // every tile is one segment of K <= kSliceSumK; of K <= kSliceFlushK
+    int stages, stage_bytes;   // the ring (set by the launcher)
+    long long wait_budget;
+};
+cudaError_t slices_init();
+cudaError_t launch_slices(const SliceArgs& a, cudaStream_t st);
+cudaError_t launch_gg_slices(const SliceGemmArgs& a, const TmaMaps& maps, cudaStream_t st);
 cudaError_t launch_pack(const PackBlock* blocks, int nb, const double* src, double* dst, int to_padded,
                         cudaStream_t st);
 int64_t dot_chunk(int64_t n);

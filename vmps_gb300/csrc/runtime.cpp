@@ -269,6 +269,68 @@ struct DevPhase {
     }
 };
 
+// device copies of one operand's slice lists and panels, and of one slice phase
+struct DevSliceOperand {
+    DBuf blocks, terms, pieces, panels, exps;
+    int npieces = 0, kcache = 32;
+    void upload(const SliceOperand& s, cudaStream_t st) {
+        npieces = (int)s.pieces.size();
+        for (const SliceBlock& b : s.blocks) kcache = std::max(kcache, std::min(kSliceCacheK, (b.K + 31) / 32 * 32));
+        upload_vec(blocks, s.blocks, st);
+        upload_vec(terms, s.terms, st);
+        upload_vec(pieces, s.pieces, st);
+        panels.alloc((size_t)s.arena.total * 2, st, true);   // zero-filled: panel padding stays zero
+        exps.alloc((size_t)(s.rows + 128) * 4, st, true);       // (the flush reads whole tiles' worth)
+    }
+    void run(const double* src, cudaStream_t st) const {
+        SliceArgs a{};
+        a.pieces = pieces.as<SlicePiece>();
+        a.blocks = blocks.as<SliceBlock>();
+        a.terms = terms.as<GTerm>();
+        a.src = src;
+        a.dst = panels.p;
+        a.exps = exps.as<int32_t>();
+        a.npieces = npieces;
+        a.kcache = kcache;
+        CK(launch_slices(a, st));
+    }
+};
+struct DevSlicePhase {
+    DBuf tiles, steps, groups, cta_tiles;
+    std::unique_ptr<TmaMaps> maps;
+    int ncta = 0, max_arows = 16, one_sum = 0, one_flush = 0;
+    void upload(const SlicePhase& ph, cudaStream_t st) {
+        ncta = ph.ncta;
+        max_arows = ph.max_arows;
+        one_sum = ph.one_sum;
+        one_flush = ph.one_flush;
+        upload_vec(tiles, ph.tiles, st);
+        upload_vec(steps, ph.steps, st);
+        upload_vec(groups, ph.groups, st);
+        upload_vec(cta_tiles, ph.cta_tiles, st);
+    }
+    void run(const DevSliceOperand& A, const DevSliceOperand& B, double* C, int* err, long long budget,
+             cudaStream_t st) const {
+        SliceGemmArgs a{};
+        a.tiles = tiles.as<SliceTile>();
+        a.steps = steps.as<SliceStep>();
+        a.groups = groups.as<SliceGroup>();
+        a.cta_tiles = cta_tiles.as<int32_t>();
+        a.ea = A.exps.as<int32_t>();
+        a.eb = B.exps.as<int32_t>();
+        a.C = C;
+        a.err = err;
+        a.ncta = ncta;
+        a.max_arows = max_arows;
+        a.one_sum = one_sum;
+        a.one_flush = one_flush;
+        a.wait_budget = budget;
+        if (ncta > 0 && (!C || !A.panels.p || !B.panels.p || !maps))
+            throw std::invalid_argument("grouped GEMM launched with an unallocated operand");
+        if (ncta > 0) CK(launch_gg_slices(a, *maps, st));
+    }
+};
+
 struct TwoSiteScratch {
     DBuf a1, a2, v, stage, pack;
     DevPhase phase;
@@ -312,6 +374,8 @@ struct DevPlan {
     DBuf ypieces;                  // PanelPiece list: the FP64 Y arena -> Y2
     int nprepX = 0, nprepZ = 0, nypieces = 0;
     std::unique_ptr<DevChunked> chunks;   // host-buffer pipeline (split plans of pivots)
+    DevSliceOperand sx, sy, sz, ss;   // FP64 slice plans
+    DevSlicePhase s1, s2;
     // split-K partial outputs (plan.splitk parts of vstride elements), one buffer per
     // output type so that the zero padding of each stays zero
     DBuf part_d, part_f;
@@ -361,6 +425,34 @@ static void encode_panel_map(CUtensorMap* m, const PanelArena& ar, const DBuf& a
     if (res != CUDA_SUCCESS)
         throw CudaFail("cuTensorMapEncodeTiled failed (" + std::to_string((int)res) + ") for a panel class of " +
                        std::to_string(c.rows) + " rows x " + std::to_string(c.kpad));
+}
+
+// A slice panel class as a 3-d tensor: 32 elements, its rows, its (K step, slice) pairs;
+// boxes of one K step's eight slices of the key's rows, 64-byte swizzle
+static void encode_slice_map(CUtensorMap* m, const PanelArena& ar, const DBuf& arena, const MapKey& k) {
+    const PanelClass& c = ar.cls.at(k.cls);
+    if (k.rows < 16 || k.rows > 256 || k.rows % 16 != 0) throw std::logic_error("TMA box rows out of range");
+    if (c.base % 64 != 0 || c.kpad % kSliceK != 0) throw std::logic_error("panel class not 128-byte aligned");
+    const cuuint64_t dims[3] = {(cuuint64_t)kSliceK, (cuuint64_t)std::max<int64_t>(c.rows, 1),
+                                (cuuint64_t)(c.kpad / kSliceK * kSlices)};
+    const cuuint64_t strides[2] = {(cuuint64_t)c.kpad * kSlices * 2, (cuuint64_t)kSliceK * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)kSliceK, (cuuint32_t)k.rows, (cuuint32_t)kSlices};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    void* base = static_cast<unsigned char*>(arena.p) + (size_t)c.base * 2;
+    const CUresult res = encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
+                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (res != CUDA_SUCCESS)
+        throw CudaFail("cuTensorMapEncodeTiled failed (" + std::to_string((int)res) + ") for a slice panel class of " +
+                       std::to_string(c.rows) + " rows x " + std::to_string(c.kpad));
+}
+static std::unique_ptr<TmaMaps> build_slice_maps(const SlicePhase& ph, const SliceOperand& A, const DBuf& Ap,
+                                                 const SliceOperand& B, const DBuf& Bp) {
+    auto m = std::make_unique<TmaMaps>();
+    std::memset(m.get(), 0, sizeof(TmaMaps));
+    for (size_t i = 0; i < ph.amaps.size(); ++i) encode_slice_map(&m->a[i], A.arena, Ap, ph.amaps[i]);
+    for (size_t i = 0; i < ph.bmaps.size(); ++i) encode_slice_map(&m->b[i], B.arena, Bp, ph.bmaps[i]);
+    return m;
 }
 
 static std::unique_ptr<TmaMaps> build_phase_maps(const PhasePlan& ph, const PanelArena& A, const DBuf& Aarena,
@@ -588,6 +680,17 @@ static void validate_tma_schedule(const PhasePlan& ph, const PanelArena& A, cons
 }
 
 static void schedule_and_validate(Plan& p, int ncta) {
+    if (p.slices) {
+        // association 0: T = op(X) Y, out = S op(Z); 1: U = Y op(Z), out = op(X) S
+        const bool xy = p.association == 0;
+        const SliceOperand &A1 = xy ? p.sx : p.sy, &B1 = xy ? p.sy : p.sz, &A2 = xy ? p.ss : p.sx, &B2 = xy ? p.sz : p.ss;
+        schedule_slices(p.s1, ncta, A1, B1);
+        schedule_slices(p.s2, ncta, A2, B2);
+        validate_slices(p.s1, A1, B1);
+        validate_slices(p.s2, A2, B2);
+        return;
+    }
+    if (!p.split) return;
     validate_tma_plan(p.p1, p.opX, p.opY, true);
     validate_tma_plan(p.p2, p.opT, p.opZ, false);
     schedule_tma(p.p1, ncta, p.opX, p.opY, p.kstep);
@@ -599,6 +702,22 @@ static void schedule_and_validate(Plan& p, int ncta) {
 // device buffers and work lists of a freshly made plan; Y is the FP64 layout
 // the per-call vector split reads
 static void plan_to_device(DevPlan& dp, const DevLayout& Y, cudaStream_t st) {
+    if (dp.plan.slices) {
+        const Plan& p = dp.plan;
+        dp.sx.upload(p.sx, st);
+        dp.sy.upload(p.sy, st);
+        dp.sz.upload(p.sz, st);
+        dp.ss.upload(p.ss, st);
+        dp.s1.upload(p.s1, st);
+        dp.s2.upload(p.s2, st);
+        dp.T.alloc((size_t)p.T.total * 8, st, true);
+        const bool xy = p.association == 0;
+        dp.s1.maps = xy ? build_slice_maps(p.s1, p.sx, dp.sx.panels, p.sy, dp.sy.panels)
+                        : build_slice_maps(p.s1, p.sy, dp.sy.panels, p.sz, dp.sz.panels);
+        dp.s2.maps = xy ? build_slice_maps(p.s2, p.ss, dp.ss.panels, p.sz, dp.sz.panels)
+                        : build_slice_maps(p.s2, p.sx, dp.sx.panels, p.ss, dp.ss.panels);
+        return;
+    }
     dp.p1.upload(dp.plan.p1, st);
     dp.p2.upload(dp.plan.p2, st);
     if (!dp.plan.split) {
@@ -627,8 +746,13 @@ static void plan_to_device(DevPlan& dp, const DevLayout& Y, cudaStream_t st) {
     }
 }
 
-// split plans: the bf16 panels of the X and scaled Z operands
+// split plans: the bf16 panels of the X and scaled Z operands; slice plans: their slices
 static void split_prepare(DevPlan& dp, const double* X, const double* Z, cudaStream_t st) {
+    if (dp.plan.slices) {
+        dp.sx.run(X, st);
+        dp.sz.run(Z, st);
+        return;
+    }
     if (!dp.plan.split) return;
     if (dp.plan.elt == 4) {
         CK(launch_prep_tf32(dp.prepX.as<PrepBlock>(), dp.nprepX, X, dp.X2.p, st));
@@ -690,6 +814,17 @@ static void run_phase_on(const DevPlan& dp, int ph, const DevPhase& d, const Pha
 }
 
 static void run_phase(const DevPlan& dp, int ph, const Operands& ops, cudaStream_t st) {
+    if (dp.plan.slices) {
+        const bool xy = dp.plan.association == 0;
+        double* T = dp.T.as<double>();
+        if (ph == 1) {
+            dp.s1.run(xy ? dp.sx : dp.sy, xy ? dp.sy : dp.sz, T, ops.err, ops.wait_budget, st);
+        } else {
+            dp.ss.run(T, st);   // the sums of first-stage products, sliced
+            dp.s2.run(xy ? dp.ss : dp.sx, xy ? dp.sz : dp.ss, ops.O, ops.err, ops.wait_budget, st);
+        }
+        return;
+    }
     if (ph == 1) run_phase_on(dp, 1, dp.p1, dp.plan.p1, ops, st);
     else run_phase_on(dp, 2, dp.p2, dp.plan.p2, ops, st);
 }
@@ -697,6 +832,7 @@ static void run_phase(const DevPlan& dp, int ph, const Operands& ops, cudaStream
 // one application of a planned contraction: (split plans) split Y, phase 1, phase 2
 static void run_plan(const DevPlan& dp, const Operands& ops, cudaStream_t st) {
     if ((ops.Yf || ops.Of) && !dp.plan.split) throw std::invalid_argument("FP32 vectors need a split plan");
+    if (dp.plan.slices) dp.sy.run(ops.Y, st);
     if (dp.plan.split && dp.plan.elt == 4) {
         CK(launch_panel_split_tf32(dp.ypieces.as<PanelPiece>(), dp.nypieces, ops.Yf ? nullptr : ops.Y, ops.Yf, dp.Y2.p,
                                    st));
@@ -737,8 +873,8 @@ static void fill_stats(const ChainSet& cs, const Plan& p, int prec, vmps_plan_st
     s->n_chains_raw = cs.n_chains_raw;
     s->n_intermediates = p.n_intermediates;
     s->n_out_blocks = p.n_out_blocks;
-    s->n_tiles_phase1 = (int64_t)p.p1.tiles.size();
-    s->n_tiles_phase2 = (int64_t)p.p2.tiles.size();
+    s->n_tiles_phase1 = (int64_t)(p.slices ? p.s1.tiles.size() : p.p1.tiles.size());
+    s->n_tiles_phase2 = (int64_t)(p.slices ? p.s2.tiles.size() : p.p2.tiles.size());
     s->flops_reference = cs.flops_reference;
     s->flops_merged = p.flops_merged;
     s->flops_phase1 = p.p1.flops;
@@ -822,8 +958,10 @@ static DevPlan& get_plan(vmps_pivot* p, int prec) {
         throw std::invalid_argument("unknown precision");
     DevPlan& dp = p->plans[prec];
     if (dp.ready) return dp;
-    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false);
-    else if (prec == VMPS_PREC_TF32X3) {
+    if (prec == VMPS_PREC_FP64) {
+        dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false);
+        schedule_and_validate(dp.plan, p->ctx->num_sms);
+    } else if (prec == VMPS_PREC_TF32X3) {
         dp.plan = make_split_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, 1, SplitTiling(), true);
         schedule_and_validate(dp.plan, p->ctx->num_sms);
     } else {
@@ -2740,11 +2878,9 @@ static DevPlan& env_plan(vmps_env* e, int prec) {
     // left: X = Abra^dagger, Y = Eold, Z = Aket;  right: X = Aket, Y = Eold, Z = Abra^dagger
     const DevLayout& X = L ? e->Bd : e->Kd;
     const DevLayout& Z = L ? e->Kd : e->Bd;
-    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
-    else {
-        dp.plan = make_split_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
-        schedule_and_validate(dp.plan, e->ctx->num_sms);
-    }
+    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L, true);
+    else dp.plan = make_split_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
+    schedule_and_validate(dp.plan, e->ctx->num_sms);
     if (e->ctx->device < 0) { dp.ready = true; return dp; }
     plan_to_device(dp, e->Ed, e->st());
     CK(cudaStreamSynchronize(e->st()));

@@ -13,6 +13,7 @@
 // chains, shares first-stage products and lays the work out as tile lists.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <set>
@@ -1039,8 +1040,262 @@ PhasePlan make_product_plan(const DevLayout& A, const DevLayout& B, const DevLay
     return ph;
 }
 
+// ===========================================================================
+// FP64 slice engine (slices.cu)
+// ===========================================================================
+namespace {
+// a block of `outer` panel rows of contraction length K; trans and ld as in SliceBlock
+int32_t add_slice_block(SliceOperand& s, int64_t outer, int64_t K, int trans, int64_t ld, const GTerm* terms, size_t n) {
+    const int32_t kp = panel_kpad(K);
+    size_t c = 0;
+    while (c < s.arena.cls.size() && s.arena.cls[c].kpad != kp) ++c;
+    if (c == s.arena.cls.size()) s.arena.cls.push_back(PanelClass{kp, 0, 0});
+    OpBlock b{};
+    b.outer = (int32_t)outer;
+    b.K = (int32_t)K;
+    b.cls = (int32_t)c;
+    b.row = (int32_t)s.arena.cls[c].rows;
+    b.pitch = kSlices * kp;
+    b.pad = (int32_t)s.rows;
+    s.arena.cls[c].rows += outer;
+    SliceBlock sb{};
+    sb.erow = b.pad;
+    sb.rows = b.outer;
+    sb.K = b.K;
+    sb.pitch = b.pitch;
+    sb.trans = trans;
+    sb.ld = (int32_t)ld;
+    sb.term_begin = (int32_t)s.terms.size();
+    sb.term_count = (int32_t)n;
+    s.terms.insert(s.terms.end(), terms, terms + n);
+    const int32_t id = (int32_t)s.op.size();
+    for (int32_t r = 0; r < b.outer; r += 32) s.pieces.push_back(SlicePiece{id, r});
+    s.rows += outer;
+    s.op.push_back(b);
+    s.blocks.push_back(sb);
+    return id;
+}
+// class matrices one after another, then every block's element offset
+void finish_slices(SliceOperand& s) {
+    int64_t cur = 0;
+    for (PanelClass& c : s.arena.cls) {
+        c.base = cur;
+        cur = (cur + kSlices * (int64_t)c.kpad * std::max<int64_t>(c.rows, 1) + 511) / 512 * 512;
+    }
+    s.arena.total = std::max<int64_t>(cur, 512);
+    for (size_t i = 0; i < s.op.size(); ++i) {
+        s.op[i].off = s.arena.cls[s.op[i].cls].base + (int64_t)s.op[i].row * s.op[i].pitch;
+        s.blocks[i].dst_off = s.op[i].off;
+    }
+}
+void add_slice_tiles(SlicePhase& ph, int64_t c_off, int64_t ldc, int64_t m, int64_t n, int32_t sb, int32_t se) {
+    for (const auto& rs : split_extent(m, 1, kSliceTileM))
+        for (const auto& cs : split_extent(n, 1, kSliceTileN)) {
+            SliceTile t{};
+            t.c_off = c_off;
+            t.ldc = (int32_t)ldc;
+            t.row0 = (int32_t)rs.first;
+            t.tm = (int32_t)rs.second;
+            t.col0 = (int32_t)cs.first;
+            t.tn = (int32_t)cs.second;
+            ph.tiles.push_back(t);
+            ph.tile_segs.push_back({sb, se});
+        }
+}
+// TMA box heights of A: the tile's rows rounded up to 16, or (fewer descriptors) 16, 32, 64 or 112
+int32_t slice_box_a(int32_t tm, bool fine) {
+    return std::min<int32_t>(kSliceTileM, fine ? std::max<int32_t>(16, (tm + 15) / 16 * 16) : box_rows_a(tm, false));
+}
+
+// FMAs or slices for an FP64 plan of `flops` whose phases would have `tiles` slice tiles.
+// VMPS_FP64_ENGINE = fma | slices | auto overrides the rule.
+//
+// FMAs run at ~0.75 TFLOP/s (1.35 us per MFLOP).  A slice tile costs ~2.7 us of one of 152
+// SMs whatever its size (0.018 us), the slices ~0.3 us per MFLOP more, and the plan two
+// launches (~8 us) more.  Whole HxVs, FMAs against slices: two-site Hubbard 141 / 158 us at
+// 55 MFLOP and 4,000 tiles, 222 / 186 at 130; one-site Hubbard 83 / 89 at 13 MFLOP, 155 / 109
+// at 68; two-site Heisenberg 87 / 80 at 7, 160 / 103 at 55; SU(2)xU(1) cylinder 109 / 113 at
+// 10, 152 / 124 at 25.
+//
+// A plan that is applied once (an environment update) would pay for the slices of all three
+// operands and for a longer list of steps: FMAs.  Whole updates, FMAs against slices: Hubbard
+// 1252 / 1291 us at 68 MFLOP, 2296 / 1999 at 500, 7654 / 3762 at 4,000; cylinder 1874 / 2155 at
+// 48, 2623 / 2554 at 280.  It is a small part of a sweep, whose split-precision HxVs round the
+// environment to FP32, so it keeps its order of summation at every size.
+bool slice_engine(double flops, double tiles, bool once) {
+    const char* v = std::getenv("VMPS_FP64_ENGINE");
+    if (v && *v && std::strcmp(v, "auto") != 0) {
+        if (!std::strcmp(v, "fma")) return false;
+        if (!std::strcmp(v, "slices")) return true;
+        throw std::invalid_argument("VMPS_FP64_ENGINE must be auto, fma or slices");
+    }
+    return !once && flops >= 18e3 * tiles + 8e6;
+}
+}  // namespace
+
+void schedule_slices(SlicePhase& ph, int ncta, const SliceOperand& A, const SliceOperand& B) {
+    const size_t nt = ph.tiles.size();
+    ph.steps.clear();
+    ph.groups.clear();
+    ph.amaps.clear();
+    ph.bmaps.clear();
+    ph.cta_tiles.assign(1, 0);
+    ph.ncta = 0;
+    ph.max_arows = 16;
+    ph.one_sum = ph.one_flush = true;
+    int64_t ends = 0;
+    if (nt == 0 || ncta <= 0) return;
+    ncta = (int)std::min<size_t>((size_t)ncta, nt);
+    // cost of a tile in K16 slices of products: a flush costs about three of them
+    std::vector<double> cost(nt);
+    bool fine = true;
+    {
+        std::set<std::pair<int32_t, int32_t>> ka;
+        for (size_t i = 0; i < nt; ++i) {
+            double c = 3;
+            for (int32_t s = ph.tile_segs[i][0]; s < ph.tile_segs[i][1]; ++s) {
+                const OpBlock& a = A.op[ph.segs[s].a];
+                c += (a.K + 15) / 16 * (ph.tiles[i].tn <= 16 ? 0.6 : 1.0) + 3.0 * ((a.K + kSliceFlushK - 1) / kSliceFlushK);
+                ka.insert({a.cls, slice_box_a(ph.tiles[i].tm, true)});
+            }
+            cost[i] = c;
+        }
+        fine = (int)ka.size() <= kMaxMapsA;
+    }
+    std::vector<size_t> order(nt);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cost[a] > cost[b]; });
+    using Load = std::pair<double, int>;
+    std::priority_queue<Load, std::vector<Load>, std::greater<Load>> heap;
+    for (int b = 0; b < ncta; ++b) heap.push({0.0, b});
+    std::vector<std::vector<size_t>> per(ncta);
+    for (size_t i : order) {
+        Load l = heap.top();
+        heap.pop();
+        per[l.second].push_back(i);
+        heap.push({l.first + cost[i], l.second});
+    }
+    auto map_of = [](std::vector<MapKey>& keys, int32_t cls, int32_t rows) {
+        for (size_t i = 0; i < keys.size(); ++i)
+            if (keys[i].cls == cls && keys[i].rows == rows) return (int32_t)i;
+        keys.push_back(MapKey{cls, rows});
+        return (int32_t)keys.size() - 1;
+    };
+    std::vector<SliceTile> tiles;
+    std::vector<std::array<int32_t, 2>> tsegs;
+    tiles.reserve(nt);
+    tsegs.reserve(nt);
+    ph.cta_tiles.assign(ncta + 1, 0);
+    for (int b = 0; b < ncta; ++b) {
+        for (size_t i : per[b]) {
+            SliceTile t = ph.tiles[i];
+            t.step0 = (int32_t)ph.steps.size();
+            t.group0 = (int32_t)ph.groups.size();
+            const int32_t ha = slice_box_a(t.tm, fine), hb = t.tn <= 16 ? 16 : 32;
+            ph.max_arows = std::max(ph.max_arows, ha);
+            for (int32_t s = ph.tile_segs[i][0]; s < ph.tile_segs[i][1]; ++s) {
+                const OpBlock& oa = A.op[ph.segs[s].a];
+                const OpBlock& ob = B.op[ph.segs[s].b];
+                const int32_t am = map_of(ph.amaps, oa.cls, ha), bm = map_of(ph.bmaps, ob.cls, hb);
+                for (int32_t k0 = 0; k0 < oa.K; k0 += kSliceK) {
+                    SliceStep st{};
+                    st.amap = am;
+                    st.bmap = bm;
+                    st.az = st.bz = k0 / kSliceK * kSlices;
+                    st.ay = oa.row + t.row0;
+                    st.by = ob.row + t.col0;
+                    st.arows = ha;
+                    const bool first = k0 % kSliceFlushK == 0;
+                    const bool last = k0 + kSliceK >= oa.K || (k0 + kSliceK) % kSliceFlushK == 0;
+                    st.flags = (oa.K - k0 <= 16 ? kSliceHalf : 0) | (first ? kSliceFirst : 0) | (last ? kSliceLast : 0) |
+                               (hb == 16 ? kSliceNarrow : 0);
+                    if (first) {
+                        const bool end = k0 + kSliceFlushK >= oa.K || (k0 + kSliceFlushK) % kSliceSumK == 0;
+                        ph.groups.push_back(SliceGroup{oa.pad + t.row0, ob.pad + t.col0, end ? kSliceSumEnd : 0, 0});
+                    }
+                    ph.steps.push_back(st);
+                }
+            }
+            t.nsteps = (int32_t)ph.steps.size() - t.step0;
+            t.ngroups = (int32_t)ph.groups.size() - t.group0;
+            const int32_t nseg = ph.tile_segs[i][1] - ph.tile_segs[i][0];
+            const int32_t klen = nseg > 0 ? A.op[ph.segs[ph.tile_segs[i][0]].a].K : 0;
+            ph.one_sum = ph.one_sum && nseg <= 1 && klen <= kSliceSumK;
+            ends += nseg;
+            for (int32_t sg = ph.tile_segs[i][0]; sg < ph.tile_segs[i][1]; ++sg)
+                ends += (A.op[ph.segs[sg].a].K - 1) / kSliceSumK;
+            ph.one_flush = ph.one_flush && klen <= kSliceFlushK;
+            tiles.push_back(t);
+            tsegs.push_back(ph.tile_segs[i]);
+        }
+        ph.cta_tiles[b + 1] = (int32_t)tiles.size();
+    }
+    // sums over several segments: each flush by itself where few of them would be joined
+    if (!ph.one_sum) ph.one_flush = (int64_t)ph.groups.size() * 3 <= ends * 4;
+    ph.tiles.swap(tiles);
+    ph.tile_segs.swap(tsegs);
+    ph.ncta = ncta;
+}
+
+void validate_slices(const SlicePhase& ph, const SliceOperand& A, const SliceOperand& B) {
+    auto need = [](bool ok, const char* what) {
+        if (!ok) throw std::logic_error(std::string("slice plan: ") + what);
+    };
+    if (ph.tiles.empty()) return;
+    need(ph.ncta > 0 && (int)ph.cta_tiles.size() == ph.ncta + 1 && ph.cta_tiles.front() == 0 &&
+             ph.cta_tiles.back() == (int32_t)ph.tiles.size(), "CTA ranges do not cover the tiles");
+    for (int b = 0; b < ph.ncta; ++b) need(ph.cta_tiles[b + 1] >= ph.cta_tiles[b], "CTA ranges out of order");
+    need((int)ph.amaps.size() <= kMaxMapsA && (int)ph.bmaps.size() <= kMaxMapsB, "too many TMA descriptors");
+    int64_t step = 0, group = 0;
+    for (size_t i = 0; i < ph.tiles.size(); ++i) {
+        const SliceTile& t = ph.tiles[i];
+        need(t.tm > 0 && t.tn > 0 && t.tm <= kSliceTileM && t.tn <= kSliceTileN && t.row0 >= 0 && t.col0 >= 0,
+             "tile shape out of range");
+        need(t.step0 == step && t.group0 == group, "tile steps not contiguous");
+        step += t.nsteps;
+        group += t.ngroups;
+        need(step <= (int64_t)ph.steps.size() && group <= (int64_t)ph.groups.size(), "tile outside the step list");
+        for (int32_t s = ph.tile_segs[i][0]; s < ph.tile_segs[i][1]; ++s) {
+            const OpBlock &a = A.op.at(ph.segs.at(s).a), &b = B.op.at(ph.segs[s].b);
+            need(a.K == b.K && a.K > 0 && t.row0 + t.tm <= a.outer && t.col0 + t.tn <= b.outer, "tile outside its operands");
+        }
+        bool open = false;
+        int ngroups = 0, k = 0;
+        for (int j = t.step0; j < t.step0 + t.nsteps; ++j) {
+            const SliceStep& s = ph.steps[j];
+            need(s.amap >= 0 && s.amap < (int)ph.amaps.size() && s.bmap >= 0 && s.bmap < (int)ph.bmaps.size(),
+                 "descriptor out of range");
+            const MapKey &ka = ph.amaps[s.amap], &kb = ph.bmaps[s.bmap];
+            need(ka.rows == s.arows && s.arows <= ph.max_arows && s.arows >= t.tm && s.arows % 16 == 0 && s.arows <= kSliceTileM &&
+                     kb.rows == (t.tn <= 16 ? 16 : 32) && ((s.flags & kSliceNarrow) != 0) == (t.tn <= 16), "TMA box");
+            const PanelClass &ca = A.arena.cls[ka.cls], &cb = B.arena.cls[kb.cls];
+            need(s.ay >= 0 && s.ay < ca.rows && s.by >= 0 && s.by < cb.rows && s.az >= 0 && s.az % kSlices == 0 &&
+                     s.bz >= 0 && s.bz % kSlices == 0 && s.az < ca.kpad / kSliceK * kSlices &&
+                     s.bz < cb.kpad / kSliceK * kSlices, "TMA coordinate outside its panel");
+            need(((s.flags & kSliceFirst) != 0) == !open, "flush groups overlap");
+            if (!open) { ++ngroups; k = 0; }
+            k += kSliceK;
+            need(k <= kSliceFlushK, "flush group longer than the exact sum");
+            open = !(s.flags & kSliceLast);
+        }
+        need(!open && ngroups == t.ngroups, "flush group without an end");
+        int sum = 0;   // flushes of the open sum
+        for (int q = t.group0; q < t.group0 + t.ngroups; ++q) {
+            const SliceGroup& gq = ph.groups[q];
+            need(gq.ea >= 0 && gq.ea + t.tm <= A.rows && gq.eb >= 0 && gq.eb + t.tn <= B.rows, "exponent rows out of range");
+            if (sum > 0) need(gq.ea == ph.groups[q - 1].ea && gq.eb == ph.groups[q - 1].eb, "sum of unequal exponents");
+            need(++sum * kSliceFlushK <= kSliceSumK, "too many flushes in a sum");
+            if (gq.flags & kSliceSumEnd) sum = 0;
+        }
+        need(sum == 0, "sum of flushes without an end");
+        if (ph.one_sum) need(t.ngroups * kSliceFlushK <= kSliceSumK, "integer sum of a tile too long");
+        if (ph.one_sum && ph.one_flush) need(t.ngroups <= 1, "more than one flush in a tile");
+    }
+    need(step == (int64_t)ph.steps.size() && group == (int64_t)ph.groups.size(), "step count mismatch");
+}
+
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z, const DevLayout& O,
-               bool transX, bool transZ) {
+               bool transX, bool transZ, bool once) {
     Plan P;
     // shapes: op(X) m x k, Y k x n, op(Z) n x p, out m x p
     auto xm = [&](int64_t x) { return transX ? X.cols[x] : X.rows[x]; };
@@ -1127,6 +1382,15 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
     }
     P.n_intermediates = (int64_t)ipairs.size();
     P.T = make_dev_layout(trows, tcols);
+    {
+        double tiles = 0;
+        auto count = [&](int64_t m, int64_t n) {
+            tiles += (double)((m + kSliceTileM - 1) / kSliceTileM) * (double)((n + kSliceTileN - 1) / kSliceTileN);
+        };
+        for (size_t j = 0; j < ipairs.size(); ++j) count(trows[j], tcols[j]);
+        for (size_t o = 0; o < O.rows.size(); ++o) count(O.rows[o], O.cols[o]);
+        P.slices = slice_engine(std::min(f_xy, f_yz), tiles, once);
+    }
 
     // ---- phase 1: T = op(X)*Y  (association 0)  or  U = Y*op(Z)  (association 1)
     PhasePlan& p1 = P.p1;
@@ -1137,7 +1401,33 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
     }
     p1.slotC = SLOT_T;
     p1.transC = false;
-    for (size_t j = 0; j < ipairs.size(); ++j) {
+    // slice engine: the operand blocks in use, made on first use
+    std::vector<int32_t> ix(X.rows.size(), -1), iy(Y.rows.size(), -1), iz(Z.rows.size(), -1);
+    auto slice_x = [&](int64_t x) {
+        const GTerm t{X.off[x], 1.0};
+        if (ix[x] < 0) ix[x] = add_slice_block(P.sx, xm(x), xk(x), transX ? 0 : 1, X.ld[x], &t, 1);
+        return ix[x];
+    };
+    auto slice_z = [&](int64_t z) {
+        const GTerm t{Z.off[z], 1.0};
+        if (iz[z] < 0) iz[z] = add_slice_block(P.sz, zp(z), zn(z), transZ ? 1 : 0, Z.ld[z], &t, 1);
+        return iz[z];
+    };
+    auto slice_y = [&](int64_t y) {   // columns of Y (association 0: B operand) or its rows (1: A operand)
+        const GTerm t{Y.off[y], 1.0};
+        const bool cols = P.association == 0;
+        if (iy[y] < 0)
+            iy[y] = add_slice_block(P.sy, cols ? Y.cols[y] : Y.rows[y], cols ? Y.rows[y] : Y.cols[y], cols ? 0 : 1, Y.ld[y], &t, 1);
+        return iy[y];
+    };
+    for (size_t j = 0; P.slices && j < ipairs.size(); ++j) {
+        const int64_t a = ipairs[j].first, b = ipairs[j].second;
+        const int32_t sb = (int32_t)P.s1.segs.size();
+        P.s1.segs.push_back(P.association == 0 ? SliceSeg{slice_x(a), slice_y(b)} : SliceSeg{slice_y(a), slice_z(b)});
+        p1.flops += 2.0 * trows[j] * tcols[j] * (P.association == 0 ? xk(a) : Y.cols[a]);
+        add_slice_tiles(P.s1, P.T.off[j], P.T.ld[j], trows[j], tcols[j], sb, sb + 1);
+    }
+    for (size_t j = 0; !P.slices && j < ipairs.size(); ++j) {
         int64_t a = ipairs[j].first, b = ipairs[j].second;
         const DevLayout& LA = P.association == 0 ? X : Y;
         const DevLayout& LB = P.association == 0 ? Y : Z;
@@ -1184,6 +1474,7 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
     while (i < order.size()) {
         const int64_t o = ch[order[i]].out;
         int32_t sb = (int32_t)p2.segs.size();
+        const int32_t ssb = (int32_t)P.s2.segs.size();
         size_t j = i;
         while (j < order.size() && ch[order[j]].out == o) {
             const int64_t other = P.association == 0 ? ch[order[j]].z : ch[order[j]].x;
@@ -1210,6 +1501,19 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
                 s.ldb = (int32_t)X.ld[other];
                 s.K = (int32_t)xk(other);
             }
+            if (P.slices) {
+                // S, the sum of the terms: A operand (rows of T) or B operand (columns of U)
+                const GTerm* tt = p2.terms.data() + s.term_begin;
+                const size_t nt = (size_t)(tend - s.term_begin);
+                if (P.association == 0)
+                    P.s2.segs.push_back(SliceSeg{add_slice_block(P.ss, O.rows[o], s.K, 1, s.lda, tt, nt), slice_z(other)});
+                else
+                    P.s2.segs.push_back(SliceSeg{slice_x(other), add_slice_block(P.ss, O.cols[o], s.K, 0, s.lda, tt, nt)});
+                p2.segs.push_back(s);   // its term count is not limited here
+                p2.segs.back().term_count = (int32_t)nt;
+                j = jj;
+                continue;
+            }
             // a segment carries at most kMaxTerms terms: longer sums become several
             // segments with the same B operand
             for (int32_t tb = s.term_begin; tb < tend; tb += kMaxTerms) {
@@ -1227,7 +1531,8 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         for (int32_t s = sb; s < se; ++s) { kk += p2.segs[s].K; kt += (double)p2.segs[s].K * p2.segs[s].term_count; }
         p2.flops += 2.0 * m * p * kk;
         P.flops_p2_unsummed += 2.0 * m * p * kt;
-        if (P.association == 0) tiles_of(p2, O.off[o], O.ld[o], m, p, sb, se);
+        if (P.slices) add_slice_tiles(P.s2, O.off[o], O.ld[o], m, p, ssb, (int32_t)P.s2.segs.size());
+        else if (P.association == 0) tiles_of(p2, O.off[o], O.ld[o], m, p, sb, se);
         else tiles_of(p2, O.off[o], O.ld[o], p, m, sb, se);
         i = j;
     }
@@ -1239,11 +1544,14 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         const int32_t sb = (int32_t)p2.segs.size();
         for (size_t o = 0; o < O.rows.size(); ++o)
             if (!seen[o]) {
-                if (P.association == 0) tiles_of(p2, O.off[o], O.ld[o], O.rows[o], O.cols[o], sb, sb);
+                if (P.slices) add_slice_tiles(P.s2, O.off[o], O.ld[o], O.rows[o], O.cols[o], 0, 0);
+                else if (P.association == 0) tiles_of(p2, O.off[o], O.ld[o], O.rows[o], O.cols[o], sb, sb);
                 else tiles_of(p2, O.off[o], O.ld[o], O.cols[o], O.rows[o], sb, sb);
             }
     }
     sort_tiles(p2);
+    if (P.slices)
+        for (SliceOperand* q : {&P.sx, &P.sy, &P.sz, &P.ss}) finish_slices(*q);
     return P;
 }
 
