@@ -21,6 +21,14 @@
 // the bytes and moves the FMAs off GB300's slow FP64 pipe.  Chunk partial sums,
 // alpha, beta and the coefficients are FP64 either way.
 //
+// What bounds the FP32 form is the FP64 work left in it, not memory: an FP64 addition or a
+// double <-> float conversion instruction holds an SM quadrant's pipe for 64 clocks per warp.  So
+// warp sums add several rows at once, the coefficients are converted once per block, and loops
+// over full chunks carry no bounds checks (more loads in flight).  547,000 elements and 45 basis
+// vectors (98 MB, 14.5 us at 6.8 TB/s), before and after, cold: lz_proj 31 -> 23 us, lz_orth
+// 43 -> 28, lz_local 17 -> 13.  A warp reading eight rows side by side instead of one after
+// another took 50 us in lz_proj: too few blocks fit an SM.
+//
 // The iteration index lives in device memory, so the HxV plan and these
 // kernels form one CUDA graph that the host replays per iteration.  Reductions
 // are deterministic: each block writes the partial sums of its element chunk,
@@ -105,17 +113,77 @@ struct LzVecOk {
     static constexpr bool value = E % LzPack<V>::W == 0;
 };
 
-// partial dot of basis row `ki` (chunk-relative) with the chunk of w staged in
-// shared memory: one warp, len valid elements, four independent accumulators
-// in the vector type, FP64 from the warp sum on.  Full chunks go by 16-byte
-// groups; the partial last chunk element by element.
+__device__ __forceinline__ double lz_f64(double x) { return x; }
+__device__ __forceinline__ double lz_f64(float x) { return f32_to_f64(x); }   // exact, integer pipe
+
+// FP64 warp sums of R values per lane (R = 2, 4, 8, 16): every lane returns the sum of row
+// lz_sum_row<R>(lane), the same bits as R calls of lz_warp_sum.  An FP64 addition holds a
+// quadrant's pipe for 64 clocks per warp whatever its lanes do, so the first log2(R) steps
+// give half of the lanes one row of a pair and half the other: 9 additions for 8 rows in
+// place of 40.
+template <int R>
+__device__ __forceinline__ int lz_sum_row(int lane) {
+    int r = 0;
+#pragma unroll
+    for (int b = 1, o = 16; b < R; b *= 2, o >>= 1) r += lane & o ? b : 0;
+    return r;
+}
+template <int R, typename T>
+__device__ __forceinline__ double lz_warp_sums(const T (&v)[R], int lane, int o = 16) {
+    if constexpr (R == 1) {
+        double s = lz_f64(v[0]);
+        for (; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    } else {
+        double h[R / 2];
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) {
+            const T mine = up ? v[2 * i + 1] : v[2 * i], other = up ? v[2 * i] : v[2 * i + 1];
+            h[i] = lz_f64(mine) + lz_f64(__shfl_xor_sync(0xffffffffu, other, o));
+        }
+        return lz_warp_sums<R / 2>(h, lane, o >> 1);
+    }
+}
+
+// FP64 sums over the block of R values per thread, the warps' sums added in warp order:
+// thread r of warp 0 returns row r.  All warps' values go through shared memory to warp 0,
+// which sums 8 R rows at once.
+template <int R, typename V>
+__device__ __forceinline__ double lz_block_sums(const V (&v)[R]) {
+    static_assert(kLzWarps == 8, "rows of one warp sum");
+    __shared__ V val[R][kLzThreads];
+    __shared__ double sum[R][kLzWarps];
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < R; ++r) val[r][threadIdx.x] = v[r];
+    __syncthreads();
+    if (threadIdx.x >= 32) return 0;
+    V x[R * kLzWarps];
+#pragma unroll
+    for (int q = 0; q < R * kLzWarps; ++q) x[q] = val[q / kLzWarps][(q % kLzWarps) * 32 + lane];
+    const double t = lz_warp_sums<R * kLzWarps>(x, lane);
+    const int row = lz_sum_row<R * kLzWarps>(lane);
+    if ((lane & (32 / (R * kLzWarps) - 1)) == 0) sum[row / kLzWarps][row % kLzWarps] = t;
+    __syncwarp();
+    double s = 0;
+    if (lane < R) {
+#pragma unroll
+        for (int q = 0; q < kLzWarps; ++q) s += sum[lane][q];
+    }
+    return s;
+}
+
+// the lane's part of the dot of basis row `ki` (chunk-relative) with the chunk of w staged in
+// shared memory: one warp, len valid elements, four independent accumulators in the vector type.
+// Full chunks go by 16-byte groups where the chunk allows; the partial last chunk element by
+// element.
 template <typename V, int E>
-__device__ __forceinline__ double lz_chunk_dot(const V* __restrict__ ki, const V* wsh, int len, int lane) {
+__device__ __forceinline__ V lz_chunk_dot(const V* __restrict__ ki, const V* wsh, int len, int lane) {
     V s[4] = {0, 0, 0, 0};
     constexpr int W = LzPack<V>::W;
-    bool done = false;
-    if constexpr (LzVecOk<V, E>::value) {
-        if (len == E * 256) {
+    if (len == E * 256) {
+        if constexpr (LzVecOk<V, E>::value) {
 #pragma unroll
             for (int t = 0; t < E * 8 / W; ++t) {
                 const int x = (lane + 32 * t) * W;
@@ -123,25 +191,55 @@ __device__ __forceinline__ double lz_chunk_dot(const V* __restrict__ ki, const V
 #pragma unroll
                 for (int q = 0; q < W; ++q) s[t & 3] = fma(a.v[q], b.v[q], s[t & 3]);
             }
-            done = true;
-        }
-    }
-    if (!done) {
+        } else {
 #pragma unroll
+            for (int t = 0; t < E * 8; ++t) s[t & 3] = fma(ki[lane + 32 * t], wsh[lane + 32 * t], s[t & 3]);
+        }
+    } else {
+#pragma unroll 4
         for (int t = 0; t < E * 8; ++t) {
             const int x = lane + 32 * t;
             if (x < len) s[t & 3] = fma(ki[x], wsh[x], s[t & 3]);
         }
     }
-    return lz_warp_sum((double)((s[0] + s[1]) + (s[2] + s[3])));
+    return (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// part[i][block] = chunk dot of basis row i, for i < m: a warp takes every eighth row, and its
+// rows' lane parts, up to eight at a time, are summed together in FP64
+template <typename V, int R>
+__device__ __forceinline__ void lz_store_sums(const V (&v)[8], int i0, int m, double* part, int nchunk) {
+    const int lane = threadIdx.x & 31;
+    V u[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) u[r] = v[r];
+    const double t = lz_warp_sums<R>(u, lane);
+    const int i = i0 + kLzWarps * lz_sum_row<R>(lane);
+    if ((lane & (32 / R - 1)) == 0 && i < m) part[(int64_t)i * nchunk + blockIdx.x] = t;
+}
+template <typename V, int E>
+__device__ __forceinline__ void lz_all_dots(const V* __restrict__ kb, int64_t ld, int m, const V* wsh, int len,
+                                            double* part, int nchunk) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i0 = warp; i0 < m; i0 += 8 * kLzWarps) {
+        V v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            v[r] = 0;
+            if (i0 + r * kLzWarps < m) v[r] = lz_chunk_dot<V, E>(kb + (int64_t)(i0 + r * kLzWarps) * ld, wsh, len, lane);
+        }
+        const int rows = (m - i0 + kLzWarps - 1) / kLzWarps;
+        if (rows == 1) lz_store_sums<V, 1>(v, i0, m, part, nchunk);
+        else if (rows == 2) lz_store_sums<V, 2>(v, i0, m, part, nchunk);
+        else if (rows <= 4) lz_store_sums<V, 4>(v, i0, m, part, nchunk);
+        else lz_store_sums<V, 8>(v, i0, m, part, nchunk);
+    }
 }
 
 template <typename V, int E>
 __global__ void __launch_bounds__(kLzThreads) lz_local_kernel(LzArgs a) {
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
-    __shared__ double red[2][kLzWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t e0 = (int64_t)blockIdx.x * (E * kLzThreads) + threadIdx.x;
     const V* K = (const V*)a.K;
     const V* w = (const V*)a.w;
@@ -157,14 +255,9 @@ __global__ void __launch_bounds__(kLzThreads) lz_local_kernel(LzArgs a) {
             if (km) s0 = fma(km[e], x, s0);
         }
     }
-    const double d0 = lz_warp_sum((double)s0), d1 = lz_warp_sum((double)s1);
-    if (lane == 0) { red[0][warp] = d0; red[1][warp] = d1; }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-        double t = 0;
-        for (int q = 0; q < kLzWarps; ++q) t += red[threadIdx.x][q];
-        a.part[(int64_t)threadIdx.x * a.nchunk + blockIdx.x] = t;
-    }
+    const V sums[2] = {s0, s1};
+    const double t = lz_block_sums<2>(sums);
+    if (threadIdx.x < 2) a.part[(int64_t)threadIdx.x * a.nchunk + blockIdx.x] = t;
     if (!lz_last_block(a.ctl + 1)) return;
     const double t0 = lz_block_row_sum(a.part, 0, a.nchunk), t1 = lz_block_row_sum(a.part, 1, a.nchunk);
     if (threadIdx.x == 0) {
@@ -179,7 +272,6 @@ __global__ void __launch_bounds__(kLzThreads) lz_proj_kernel(LzArgs a) {
     __shared__ __align__(16) V wsh[E * kLzThreads];   // this block's chunk of w after the local step
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t cb = (int64_t)blockIdx.x * (E * kLzThreads);
     const int len = (int)(a.n - cb < E * kLzThreads ? a.n - cb : E * kLzThreads);
     const V c0 = (V)a.cl[0], c1 = (V)a.cl[1];
@@ -223,11 +315,8 @@ __global__ void __launch_bounds__(kLzThreads) lz_proj_kernel(LzArgs a) {
         }
     }
     __syncthreads();
-    // one warp per basis row: d_i partial over this chunk (summed by lz_coef)
-    for (int i = warp; i <= j; i += kLzWarps) {
-        const double t = lz_chunk_dot<V, E>(K + (int64_t)i * a.ld + cb, wsh, len, lane);
-        if (lane == 0) a.part[(int64_t)i * a.nchunk + blockIdx.x] = t;
-    }
+    // d_i partials over this chunk (summed by lz_coef)
+    lz_all_dots<V, E>(K + cb, a.ld, j + 1, wsh, len, a.part, a.nchunk);
 }
 
 // d_i = sum over chunks of lz_proj's partials, one block per basis row
@@ -244,8 +333,10 @@ template <typename V, int E>
 __global__ void __launch_bounds__(kLzThreads) lz_orth_kernel(LzArgs a) {
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
-    __shared__ double red[kLzWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the coefficients in the vector type, converted once per block
+    __shared__ V csh[kLzMaxIter];
+    for (int i = threadIdx.x; i <= j; i += kLzThreads) csh[i] = (V)a.coef[i];
+    __syncthreads();
     const int64_t e0 = (int64_t)blockIdx.x * (E * kLzThreads) + threadIdx.x;
     const V* K = (const V*)a.K;
     V* w = (V*)a.w;
@@ -259,10 +350,10 @@ __global__ void __launch_bounds__(kLzThreads) lz_orth_kernel(LzArgs a) {
         LzPack<V> wr[E / W];
 #pragma unroll
         for (int u = 0; u < E / W; ++u) wr[u] = lz_ld16(w + cb + (threadIdx.x + u * kLzThreads) * W);
-#pragma unroll 2
+#pragma unroll(E / W >= 4 ? 2 : 8 / (E / W))
         for (int i = 0; i <= j; ++i) {
             const V* ki = K + (int64_t)i * a.ld + cb;
-            const V d = (V)a.coef[i];
+            const V d = csh[i];
 #pragma unroll
             for (int u = 0; u < E / W; ++u) {
                 const LzPack<V> kv = lz_ld16(ki + (threadIdx.x + u * kLzThreads) * W);
@@ -286,14 +377,24 @@ __global__ void __launch_bounds__(kLzThreads) lz_orth_kernel(LzArgs a) {
             const int64_t e = e0 + u * kLzThreads;
             wr[u] = e < a.n ? w[e] : V(0);
         }
-#pragma unroll 4
-        for (int i = 0; i <= j; ++i) {
-            const V* ki = K + (int64_t)i * a.ld;
-            const V d = (V)a.coef[i];
+        if (cb + E * kLzThreads <= a.n) {
+#pragma unroll(E >= 4 ? 2 : 8)
+            for (int i = 0; i <= j; ++i) {
+                const V* ki = K + (int64_t)i * a.ld + e0;
+                const V d = csh[i];
 #pragma unroll
-            for (int u = 0; u < E; ++u) {
-                const int64_t e = e0 + u * kLzThreads;
-                if (e < a.n) wr[u] = fma(-d, ki[e], wr[u]);
+                for (int u = 0; u < E; ++u) wr[u] = fma(-d, ki[u * kLzThreads], wr[u]);
+            }
+        } else {
+#pragma unroll 4
+            for (int i = 0; i <= j; ++i) {
+                const V* ki = K + (int64_t)i * a.ld;
+                const V d = csh[i];
+#pragma unroll
+                for (int u = 0; u < E; ++u) {
+                    const int64_t e = e0 + u * kLzThreads;
+                    if (e < a.n) wr[u] = fma(-d, ki[e], wr[u]);
+                }
             }
         }
 #pragma unroll
@@ -305,14 +406,9 @@ __global__ void __launch_bounds__(kLzThreads) lz_orth_kernel(LzArgs a) {
             }
         }
     }
-    const double ds = lz_warp_sum((double)s);
-    if (lane == 0) red[warp] = ds;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0;
-        for (int q = 0; q < kLzWarps; ++q) t += red[q];
-        a.part[blockIdx.x] = t;
-    }
+    const V sums[1] = {s};
+    const double t = lz_block_sums<1>(sums);
+    if (threadIdx.x == 0) a.part[blockIdx.x] = t;
     if (!lz_last_block(a.ctl + 3)) return;
     const double ww = lz_block_row_sum(a.part, 0, a.nchunk);
     if (threadIdx.x == 0) {
@@ -339,15 +435,17 @@ __global__ void lz_next_kernel(LzArgs a) {
     V* k = (V*)a.K + (int64_t)jn * a.ld;
     const V* w = (const V*)a.w;
     V* q = (V*)a.q;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
-        const V v = w[i] * s;
-        k[i] = v;
-        q[i] = v;
+    constexpr int W = LzPack<V>::W;   // rows and vectors start on 16 bytes
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = t0; i < a.n / W; i += nt) {
+        LzPack<V> v = lz_ld16(w + i * W);
+#pragma unroll
+        for (int q = 0; q < W; ++q) v.v[q] *= s;
+        lz_st16(k + i * W, v);
+        lz_st16(q + i * W, v);
     }
+    for (int64_t i = a.n / W * W + t0; i < a.n; i += nt) k[i] = q[i] = w[i] * s;
 }
-
-__device__ __forceinline__ double lz_f64(double x) { return x; }
-__device__ __forceinline__ double lz_f64(float x) { return f32_to_f64(x); }   // exact, integer pipe
 
 // y[e] = sum_{i < m} c[i] K_i[e] in FP64 (Ritz vectors and corrections)
 template <typename V>
@@ -367,7 +465,6 @@ __global__ void __launch_bounds__(kLzThreads) lz_mdot_kernel(const V* __restrict
                                                               const double* __restrict__ r,
                                                               double* __restrict__ part, int nchunk) {
     __shared__ __align__(16) V rsh[E * kLzThreads];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t cb = (int64_t)blockIdx.x * (E * kLzThreads);
     const int len = (int)(n - cb < E * kLzThreads ? n - cb : E * kLzThreads);
 #pragma unroll
@@ -376,10 +473,7 @@ __global__ void __launch_bounds__(kLzThreads) lz_mdot_kernel(const V* __restrict
         rsh[x] = (V)(x < len ? r[cb + x] : 0.0);
     }
     __syncthreads();
-    for (int i = warp; i < m; i += kLzWarps) {
-        const double t = lz_chunk_dot<V, E>(K + (int64_t)i * ld + cb, rsh, len, lane);
-        if (lane == 0) part[(int64_t)i * nchunk + blockIdx.x] = t;
-    }
+    lz_all_dots<V, E>(K + cb, ld, m, rsh, len, part, nchunk);
 }
 
 // out[i] = sum over chunks of part[i], i < rows, one block per row
@@ -412,7 +506,6 @@ __global__ void __launch_bounds__(kLzThreads) cheb_step_kernel(ChebArgs a) {
     const int64_t base = (int64_t)k * a.vs;
     const int64_t pe = a.pbeg[pj + 1];
     const int64_t e0 = a.pbeg[pj] + (int64_t)blockIdx.x * (E * kLzThreads) + threadIdx.x;
-    __shared__ double red[2][kLzWarps];
     double s0 = 0, s1 = 0;
 #pragma unroll
     for (int u = 0; u < E; ++u) {
@@ -425,15 +518,9 @@ __global__ void __launch_bounds__(kLzThreads) cheb_step_kernel(ChebArgs a) {
             s1 = fma(v, x, s1);
         }
     }
-    s0 = lz_warp_sum(s0);
-    s1 = lz_warp_sum(s1);
-    if (lane == 0) { red[0][warp] = s0; red[1][warp] = s1; }
-    __syncthreads();
-    if (threadIdx.x < 2) {
-        double t = 0;
-        for (int q = 0; q < kLzWarps; ++q) t += red[threadIdx.x][q];
-        a.part[(((int64_t)k * a.nparts + pj) * 2 + threadIdx.x) * a.nchunk + blockIdx.x] = t;
-    }
+    const double sums[2] = {s0, s1};
+    const double t = lz_block_sums<2>(sums);
+    if (threadIdx.x < 2) a.part[(((int64_t)k * a.nparts + pj) * 2 + threadIdx.x) * a.nchunk + blockIdx.x] = t;
     // last block of the whole grid
     __shared__ bool last;
     __threadfence();
