@@ -38,7 +38,9 @@ namespace vmps {
 // 0.76 to 0.43 ms and from 17.9 to 16.3 ms, the FP64 pipe bounding both.  Small
 // ones are bound by the latency of the segment chain, so the segments and terms
 // of a tile come to shared memory first and each K chunk's loads are issued one
-// chunk ahead.
+// chunk ahead.  Several right-hand sides share a launch (blockIdx.y): one launch
+// of 16 vectors of the two-site Hubbard pivot at D = 256 (5.2 MFLOP each) in place
+// of 16 launches, each too short to fill the chip.
 // ===========================================================================
 namespace f64k {
 constexpr int T = kTileMax, NT = 128, BK = 16, LD = T + 1;
@@ -52,8 +54,8 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
     __shared__ GSeg sseg[SEGS];
     __shared__ GTerm sterm[SEGS * kMaxTerms];
     const GTile tile = g.tiles[blockIdx.x];
-    const double* __restrict__ A = (const double*)g.A;
-    const double* __restrict__ B = (const double*)g.B;
+    const double* __restrict__ A = (const double*)g.A + blockIdx.y * g.strideA;
+    const double* __restrict__ B = (const double*)g.B + blockIdx.y * g.strideB;
     const int tid = threadIdx.x, tm = tile.tm, tn = tile.tn, ne = tm * tn;
     const bool tA = g.transA, tB = g.transB;
     // the output elements of this thread, column by column; a second one for tiles of more than 128
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
             buf ^= 1;
         }
     }
-    double* __restrict__ C = (double*)g.C + tile.c_off;
+    double* __restrict__ C = (double*)g.C + blockIdx.y * g.strideC + tile.c_off;
     auto put = [&](int i, int j, double x) {
         const int64_t gr = tile.row0 + i, gc = tile.col0 + j;
         C[g.transC ? gc + gr * tile.ldc : gr + gc * tile.ldc] = x;
@@ -538,7 +540,8 @@ cudaError_t kernels_init() {
 
 cudaError_t launch_gg64(const GGArgs& a, cudaStream_t st) {
     if (a.ntiles <= 0) return cudaSuccess;
-    gg_fp64_kernel<<<a.ntiles, f64k::NT, 0, st>>>(a);
+    if (a.nrhs < 1 || a.nrhs > 65535) return cudaErrorInvalidValue;
+    gg_fp64_kernel<<<dim3(a.ntiles, a.nrhs), f64k::NT, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -22,6 +22,10 @@ struct GGArgs {
     int ntiles;
     int transA, transB, transC;
     int64_t vstride;   // multi-RHS phase 2: element stride between the output vectors
+    // FP64 engine: right-hand sides of one launch and the element strides of the operands between
+    // them (0: shared)
+    int nrhs = 1;
+    int64_t strideA = 0, strideB = 0, strideC = 0;
     long long wait_budget;   // tcgen05 engine: clock cycles a main-loop barrier wait may take (0: ~2 s)
 };
 

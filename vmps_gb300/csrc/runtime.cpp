@@ -608,6 +608,11 @@ struct Operands {
     // pivots with an excited-state projector: applied after the second phase
     const PenaltyArgs* pen = nullptr;
     long long wait_budget = 0;   // tcgen05 engine main-loop wait budget (cycles, 0: default)
+    // FP64 FMA plans: right-hand sides in one launch, vectors vstride elements apart, their
+    // first-stage products in T, one plan's T after another (null: the plan's own, one vector)
+    int nrhs = 1;
+    int64_t vstride = 0;
+    double* T = nullptr;
 };
 
 // Invariants the tcgen05 engine relies on, checked on the host once per plan:
@@ -774,19 +779,22 @@ static void run_phase_on(const DevPlan& dp, int ph, const DevPhase& d, const Pha
     a.err = ops.err;
     a.wait_budget = ops.wait_budget;
     if (!dp.plan.split) {
-        auto slot = [&](int s) -> const void* {
+        if (ops.nrhs > 1 && !ops.T) throw std::invalid_argument("several right-hand sides without their first-stage buffer");
+        auto slot = [&](int s, int64_t& stride) -> const void* {
+            stride = s == SLOT_Y || s == SLOT_OUT ? ops.vstride : s == SLOT_T ? dp.plan.T.total : 0;
             switch (s) {
                 case SLOT_X: return ops.X;
                 case SLOT_Y: return ops.Y;
                 case SLOT_Z: return ops.Z;
                 case SLOT_OUT: return ops.O;
-                case SLOT_T: return dp.T.p;
+                case SLOT_T: return ops.T ? ops.T : dp.T.p;
             }
             return nullptr;
         };
-        a.A = slot(h.slotA);
-        a.B = slot(h.slotB);
-        a.C = const_cast<void*>(slot(h.slotC));
+        a.nrhs = ops.nrhs;
+        a.A = slot(h.slotA, a.strideA);
+        a.B = slot(h.slotB, a.strideB);
+        a.C = const_cast<void*>(slot(h.slotC, a.strideC));
         // every operand of a non-empty phase must be a live device buffer
         if (d.ntiles > 0 && (!a.C || !a.tiles || !a.segs || !a.terms || (!h.segs.empty() && (!a.A || !a.B))))
             throw std::invalid_argument("grouped GEMM launched with an unallocated operand");
@@ -849,6 +857,45 @@ static void run_plan(const DevPlan& dp, const Operands& ops, cudaStream_t st) {
         PenaltyArgs a = *ops.pen;
         a.nrhs = dp.plan.nrhs;
         CK(launch_penalty(a, ops.Y, ops.Yf, ops.O, ops.Of, st));
+    }
+}
+
+// Single-vector plans applied to nrhs vectors (ops.Y and ops.O: the first, the others vstride
+// elements apart).  An FP64 FMA plan takes as many in a launch as `T` holds first-stage buffers
+// for: at D = 256 a launch of one vector of the two-site Hubbard pivot runs 13 us for 2.6 MFLOP.
+static void run_plan_rhs(const DevPlan& dp, Operands ops, int nrhs, int64_t vstride, const DBuf& T, cudaStream_t st) {
+    const int64_t tbytes = std::max<int64_t>(dp.plan.T.total, 1) * 8;
+    const bool fma = !dp.plan.split && !dp.plan.slices;
+    const int batch = fma && T.p ? (int)std::min<int64_t>(nrhs, std::max<int64_t>(1, (int64_t)T.bytes / tbytes)) : 1;
+    const double* Y = ops.Y;
+    double* O = ops.O;
+    const PenaltyArgs* pen = ops.pen;
+    if (batch > 1) ops.pen = nullptr;
+    for (int k = 0; k < nrhs; k += batch) {
+        ops.Y = Y + (int64_t)k * vstride;
+        ops.O = O + (int64_t)k * vstride;
+        ops.nrhs = std::min(batch, nrhs - k);
+        ops.vstride = vstride;
+        ops.T = batch > 1 ? T.as<double>() : nullptr;
+        run_plan(dp, ops, st);
+    }
+    if (batch > 1 && pen && pen->npen > 0)
+        for (int k = 0; k < nrhs; ++k) {
+            PenaltyArgs a = *pen;
+            a.nrhs = 1;
+            CK(launch_penalty(a, Y + (int64_t)k * vstride, nullptr, O + (int64_t)k * vstride, nullptr, st));
+        }
+}
+// first-stage buffers for run_plan_rhs: for every vector, at most 512 MiB, none where the device
+// has no room (the vectors then go one by one through the plan's own)
+constexpr int64_t kRhsBytes = int64_t(512) << 20;
+static void alloc_rhs(DBuf& T, const DevPlan& dp, int nrhs, cudaStream_t st) {
+    const int64_t tbytes = std::max<int64_t>(dp.plan.T.total, 1) * 8;
+    const int64_t m = std::min<int64_t>(nrhs, kRhsBytes / tbytes);
+    if (dp.plan.split || dp.plan.slices || m < 2) return;
+    try {
+        T.alloc((size_t)(m * tbytes), st, false);
+    } catch (const std::bad_alloc&) {
     }
 }
 
@@ -1805,7 +1852,13 @@ int vmps_hxv_multi(vmps_pivot* p, const double* vin, double* vout, int nrhs, int
         ops.O = dout;
         run_plan(dp, ops, st);
     } else {
-        for (int k = 0; k < nrhs; ++k) pivot_hxv_dev(p, prec, din + (int64_t)k * n, dout + (int64_t)k * n);
+        DevPlan& dp = get_plan(p, prec);
+        DBuf T;
+        alloc_rhs(T, dp, nrhs, st);
+        Operands ops = pivot_ops(p);
+        ops.Y = din;
+        ops.O = dout;
+        run_plan_rhs(dp, ops, nrhs, n, T, st);
     }
     for (int k = 0; k < nrhs; ++k)
         pack_out(p->ctx, p->dPack, p->npack, dout + (int64_t)k * n, dim, p->stage_out, vout + (int64_t)k * dim, st);
@@ -2590,8 +2643,8 @@ extern "C" int vmps_spectral_bounds(vmps_pivot* p, const double* v, int iters, d
 // t_{n+1} = 2 H~ t_n - t_{n-1} of the reference's polyIter / polyCompress
 // (DmrgLinearAlgebra.h:550-566, solvers/MpsCompressor.h:1372-1564) on the
 // pivot, with H~ = (H - b)/a.  One step is one CUDA graph: the HxV of all
-// right-hand sides (split precision: one grouped multi-RHS launch pair; FP64:
-// the plain HxV per vector) and cheb_step_kernel (update and FP64 moments).
+// right-hand sides (split precision: one grouped multi-RHS launch pair; FP64: one
+// launch pair by FMAs, the plain HxV per vector by slices) and cheb_step_kernel (update and FP64 moments).
 // The three vector buffers rotate, so three graphs cover every step.
 // the moments of nrhs start vectors, per part (block ranges [part_blocks[j], part_blocks[j+1])
 // of the vector layout; nparts 1 with part_blocks null: the whole vector)
@@ -2621,11 +2674,12 @@ static int chebyshev_moments(vmps_pivot* p, const double* v0, int nrhs, int nmom
     auto t0 = std::chrono::steady_clock::now();
     cudaStream_t st = p->st();
     // BF16x3: one grouped launch pair for all right-hand sides; FP64 and 3xTF32: the
-    // single-vector plan once per right-hand side
+    // single-vector plan (run_plan_rhs)
     DevPlan& dp = prec == VMPS_PREC_BF16X3 ? get_multi_plan(p, nrhs) : get_plan(p, prec);
     const int64_t dim = p->Vt.total, n = p->Vd.total;
     const size_t vbytes = (size_t)nrhs * n * 8;
-    DBuf B[3], Wb, part, mud, ctl;
+    DBuf B[3], Wb, part, mud, ctl, T;
+    alloc_rhs(T, dp, nrhs, st);
     for (DBuf& x : B) x.alloc(vbytes, st, true);
     Wb.alloc(vbytes, st, true);
     int64_t longest = 0;
@@ -2670,11 +2724,9 @@ static int chebyshev_moments(vmps_pivot* p, const double* v0, int nrhs, int nmom
                 ops.O = Wb.as<double>();
                 run_plan(dp, ops, st);
             } else {
-                for (int k = 0; k < nrhs; ++k) {
-                    ops.Y = c.tn + (int64_t)k * n;
-                    ops.O = Wb.as<double>() + (int64_t)k * n;
-                    run_plan(dp, ops, st);
-                }
+                ops.Y = c.tn;
+                ops.O = Wb.as<double>();
+                run_plan_rhs(dp, ops, nrhs, n, T, st);
             }
             CK(launch_cheb_step(c, sh.per_thread, st));
         } catch (...) {
