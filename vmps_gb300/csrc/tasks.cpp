@@ -873,6 +873,31 @@ void add_tiles(PhasePlan& ph, int64_t c_off, int64_t ldc, int64_t m, int64_t n, 
         }
 }
 
+// FP64 tiles of a phase that leaves SMs idle: those of more than 128 elements are halved, so that
+// every thread has one element and a K chunk takes half as long (16 FMAs, each holding a quadrant's
+// pipe for 64 clocks, in place of 32).  Up to one tile per SM: beyond it the halves of two tiles
+// would share an SM and the time would stay.  One-site Heisenberg HxV at D = 64 (20 to 80 tiles):
+// 61 -> 54 us; the transfer solve at 256 multiplets (63 to 132 tiles, 4 launches an iteration):
+// 222 -> 192 us an iteration.
+void halve_tiles(PhasePlan& ph) {
+    constexpr size_t kFew = 152;
+    if (ph.tiles.size() > kFew) return;
+    std::vector<GTile> out;
+    for (const GTile& t : ph.tiles) {
+        if (t.tm * t.tn <= 128) {
+            out.push_back(t);
+            continue;
+        }
+        GTile a = t, b = t;   // tm <= 16, so tn > 8
+        a.tn = t.tn / 2;
+        b.col0 += a.tn;
+        b.tn -= a.tn;
+        out.push_back(a);
+        out.push_back(b);
+    }
+    ph.tiles.swap(out);
+}
+
 // order tiles by descending work so that the hardware block scheduler runs the
 // largest first (longest-processing-time list scheduling)
 void sort_tiles(PhasePlan& ph) {
@@ -1036,6 +1061,7 @@ PhasePlan make_product_plan(const DevLayout& A, const DevLayout& B, const DevLay
         }
         add_tiles(ph, C.off[k], C.ld[k], C.rows[k], C.cols[k], sb, (int32_t)ph.segs.size(), kTileMax, kTileMax, 1, 1);
     }
+    halve_tiles(ph);
     sort_tiles(ph);
     return ph;
 }
@@ -1445,6 +1471,7 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         p1.flops += 2.0 * trows[j] * tcols[j] * K;
         tiles_of(p1, P.T.off[j], P.T.ld[j], trows[j], tcols[j], sb, sb + 1);
     }
+    halve_tiles(p1);
     sort_tiles(p1);
 
     // ---- phase 2
@@ -1549,6 +1576,7 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
                 else tiles_of(p2, O.off[o], O.ld[o], O.cols[o], O.rows[o], sb, sb);
             }
     }
+    halve_tiles(p2);
     sort_tiles(p2);
     if (P.slices)
         for (SliceOperand* q : {&P.sx, &P.sy, &P.sz, &P.ss}) finish_slices(*q);
