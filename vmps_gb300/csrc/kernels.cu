@@ -329,69 +329,124 @@ __global__ void pack_kernel(const PackBlock* blocks, int nb, const double* __res
 
 // partial dot products: fixed chunking -> deterministic two-pass reduction
 constexpr int kDotThreads = 256;
+// sum over the block, thread t + w added to thread t for w = 128 .. 1 (valid in thread 0)
+__device__ __forceinline__ double block_tree_sum(double s) {
+    __shared__ double red[kDotThreads];
+    red[threadIdx.x] = s;
+    __syncthreads();
+#pragma unroll
+    for (int w = kDotThreads / 2; w >= 32; w >>= 1) {
+        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x < 32) {
+        s = red[threadIdx.x];
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+    }
+    return s;
+}
 __global__ void dot_partial_kernel(const double* __restrict__ x, const double* __restrict__ y, int64_t n,
                                    int64_t chunk, double* __restrict__ part) {
-    __shared__ double red[kDotThreads];
     const int64_t b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
     double s = 0;
+#pragma unroll 8
     for (int64_t i = b0 + threadIdx.x; i < b1; i += kDotThreads) s = fma(x[i], y[i], s);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = kDotThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+    s = block_tree_sum(s);
+    if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 __global__ void sum_partial_kernel(const double* __restrict__ part, int np, double* __restrict__ out) {
-    __shared__ double red[kDotThreads];
     double s = 0;
     for (int i = threadIdx.x; i < np; i += kDotThreads) s += part[i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = kDotThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = red[0];
+    s = block_tree_sum(s);
+    if (threadIdx.x == 0) *out = s;
 }
-// many dots at once: out[j] = <V_j, w> for j < nv (V row-major [nv][n]); partials [nv][nchunk]
-__global__ void mdot_partial_kernel(const double* __restrict__ V, int64_t n, const double* __restrict__ w,
-                                    int64_t chunk, int nchunk, double* __restrict__ part) {
-    __shared__ double red[kDotThreads];
-    const int j = blockIdx.y;
+
+// ---- GMRES of the transfer operator ---------------------------------------------------------
+// An Arnoldi step of these short vectors (13,000 elements for 256 multiplets) is a chain of
+// launches of a few microseconds each, so the sums of partials and the dot weights are folded into
+// the kernels around them: 6 launches in place of 13, with the same roundings.  The weighted vector
+// r = wm * w is formed where w is written: formed in the dots, it took two more FP64 operations
+// per element and basis row (an operation holds an SM quadrant's pipe for 64 clocks per warp).
+//
+// part[j][chunk] of <V_j, r>, j < nv (V row-major [nv][n])
+__global__ void __launch_bounds__(kDotThreads) arnoldi_dot_kernel(const double* __restrict__ V, int64_t n,
+                                                                  const double* __restrict__ r, int64_t chunk,
+                                                                  int nchunk, double* __restrict__ part) {
     const int64_t b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
-    const double* v = V + (int64_t)j * n;
+    const double* v = V + (int64_t)blockIdx.y * n;
     double s = 0;
-    for (int64_t i = b0 + threadIdx.x; i < b1; i += kDotThreads) s = fma(v[i], w[i], s);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int ww = kDotThreads / 2; ww > 0; ww >>= 1) {
-        if (threadIdx.x < ww) red[threadIdx.x] += red[threadIdx.x + ww];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[(int64_t)j * nchunk + blockIdx.x] = red[0];
+#pragma unroll 16
+    for (int64_t i = b0 + threadIdx.x; i < b1; i += kDotThreads) s = fma(v[i], r[i], s);
+    s = block_tree_sum(s);
+    if (threadIdx.x == 0) part[(int64_t)blockIdx.y * nchunk + blockIdx.x] = s;
+}
+// the sum of nchunk <= 32 partials in the order of block_tree_sum (which adds zeros to them)
+__device__ __forceinline__ double partial_tree_sum(const double* __restrict__ p, int nchunk) {
+    double t[32];
+#pragma unroll
+    for (int c = 0; c < 32; ++c) t[c] = c < nchunk ? 0.0 + p[c] : 0.0;
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1)
+        if (w < nchunk) {
+#pragma unroll
+            for (int c = 0; c < w; ++c) t[c] += t[c + w];
+        }
+    return t[0];
 }
 __global__ void msum_partial_kernel(const double* __restrict__ part, int nchunk, double* __restrict__ out) {
-    __shared__ double red[kDotThreads];
-    const int j = blockIdx.x;
     double s = 0;
-    for (int i = threadIdx.x; i < nchunk; i += kDotThreads) s += part[(int64_t)j * nchunk + i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = kDotThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[j] = red[0];
+    for (int i = threadIdx.x; i < nchunk; i += kDotThreads) s += part[(int64_t)blockIdx.x * nchunk + i];
+    s = block_tree_sum(s);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
 }
-// w -= sum_j coef[j] V_j
-__global__ void mgs_update_kernel(const double* __restrict__ V, int nv, int64_t n, const double* __restrict__ coef,
-                                  double* __restrict__ w) {
+// w -= sum_j coef[j] V_j, r = wm * w; part set: coef[j] is summed here from nchunk <= 32 partials by every
+// block, and stored by the first
+__global__ void __launch_bounds__(256) arnoldi_update_kernel(const double* __restrict__ V, int nv, int64_t n,
+                                                             const double* __restrict__ part, int nchunk, double* coef,
+                                                             const double* __restrict__ wm, double* __restrict__ w,
+                                                             double* __restrict__ r) {
+    extern __shared__ double c[];
+    for (int j = threadIdx.x; j < nv; j += blockDim.x) {
+        const double x = part ? partial_tree_sum(part + (int64_t)j * nchunk, nchunk) : coef[j];
+        c[j] = -x;
+        if (part && blockIdx.x == 0) coef[j] = x;
+    }
+    __syncthreads();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double s = w[i];
-        for (int j = 0; j < nv; ++j) s = fma(-coef[j], V[(int64_t)j * n + i], s);
+#pragma unroll 8
+        for (int j = 0; j < nv; ++j) s = fma(c[j], V[(int64_t)j * n + i], s);
         w[i] = s;
+        r[i] = wm[i] * s;
+    }
+}
+// out[0] = <w, r>, the partials summed by the last block (out[4]: its counter, zero between
+// launches)
+__global__ void __launch_bounds__(kDotThreads) arnoldi_norm_kernel(const double* __restrict__ w,
+                                                                   const double* __restrict__ r, int64_t n, int64_t chunk,
+                                                                   double* part, double* out) {
+    const int64_t b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
+    double s = 0;
+#pragma unroll 16
+    for (int64_t i = b0 + threadIdx.x; i < b1; i += kDotThreads) s = fma(w[i], r[i], s);
+    s = block_tree_sum(s);
+    unsigned* count = reinterpret_cast<unsigned*>(out + 4);
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = s;
+        __threadfence();
+        last = atomicAdd(count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    s = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kDotThreads) s += __ldcg(part + i);
+    s = block_tree_sum(s);
+    if (threadIdx.x == 0) {
+        out[0] = s;
+        *count = 0;
     }
 }
 __global__ void axpy_kernel(double a, const double* __restrict__ x, double* __restrict__ y, int64_t n) {
@@ -403,9 +458,10 @@ __global__ void hadamard_kernel(const double* __restrict__ a, const double* __re
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = a[i] * b[i];
 }
-__global__ void scale_kernel(double a, double* __restrict__ x, int64_t n) {
+// y = a x (y = x allowed)
+__global__ void scale_kernel(double a, const double* x, double* y, int64_t n) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        x[i] *= a;
+        y[i] = x[i] * a;
 }
 // y = sum_j c[j] V_j  (Ritz vector assembly)
 __global__ void combine_kernel(const double* __restrict__ V, int nv, int64_t n, const double* __restrict__ c,
@@ -484,38 +540,49 @@ __global__ void pen_add_kernel(PenaltyArgs a, TO* __restrict__ out) {
 // VUMPS transfer operator pieces
 // ---------------------------------------------------------------------------
 // part[b] = w_b * sum_ij V[i + j*v_ld] * LR[j + i*lr_ld]  (the trace of a block product)
-__global__ void trace_pairs_kernel(const TracePair* __restrict__ tp, int n, const double* __restrict__ V,
-                                   const double* __restrict__ LR, double* __restrict__ part) {
-    __shared__ double red[kDotThreads];
+__global__ void __launch_bounds__(kDotThreads) trace_pairs_kernel(const TracePair* __restrict__ tp, int n,
+                                                                  const double* __restrict__ V,
+                                                                  const double* __restrict__ LR, double* __restrict__ part) {
     for (int b = blockIdx.x; b < n; b += gridDim.x) {
         const TracePair p = tp[b];
         double s = 0;
+#pragma unroll 8
         for (int e = threadIdx.x; e < p.rows * p.cols; e += kDotThreads) {
             const int j = e / p.rows, i = e - j * p.rows;
             s = fma(V[p.v_off + i + (int64_t)j * p.v_ld], LR[p.lr_off + j + (int64_t)i * p.lr_ld], s);
         }
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = kDotThreads / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) part[b] = p.weight * red[0];
+        s = block_tree_sum(s);
+        if (threadIdx.x == 0) part[b] = p.weight * s;
         __syncthreads();
     }
 }
 
-// out[block] = V[block] - T[block] + (*s) * identity, per matched block pair
-__global__ void transfer_combine_kernel(const CombineBlock* __restrict__ cb, int n, const double* __restrict__ V,
-                                        const double* __restrict__ T, double* __restrict__ out,
-                                        const double* __restrict__ s) {
-    const double sc = *s;
+// out[block] = V[block] - T[block] + s * identity, per matched block pair, s the sum of the np trace
+// partials (every block sums them: cheaper than a launch); r set: r = wm * out there as well.
+// gridDim.y blocks share a pair
+__global__ void __launch_bounds__(kDotThreads) transfer_combine_kernel(const CombineBlock* __restrict__ cb, int n,
+                                                                       const double* __restrict__ V,
+                                                                       const double* __restrict__ T,
+                                                                       double* __restrict__ out,
+                                                                       const double* __restrict__ part, int np,
+                                                                       const double* __restrict__ wm,
+                                                                       double* __restrict__ r) {
+    __shared__ double sc_;
+    double t = 0;
+    for (int i = threadIdx.x; i < np; i += kDotThreads) t += part[i];
+    t = block_tree_sum(t);
+    if (threadIdx.x == 0) sc_ = t;
+    __syncthreads();
+    const double sc = sc_;
     for (int b = blockIdx.x; b < n; b += gridDim.x) {
         const CombineBlock c = cb[b];
-        for (int e = threadIdx.x; e < c.rows * c.cols; e += blockDim.x) {
+#pragma unroll 4
+        for (int e = blockIdx.y * kDotThreads + threadIdx.x; e < c.rows * c.cols; e += gridDim.y * kDotThreads) {
             const int j = e / c.rows, i = e - j * c.rows;
             const int64_t vo = c.v_off + i + (int64_t)j * c.v_ld;
-            out[vo] = V[vo] - T[c.t_off + i + (int64_t)j * c.t_ld] + (i == j ? sc : 0.0);
+            const double x = V[vo] - T[c.t_off + i + (int64_t)j * c.t_ld] + (i == j ? sc : 0.0);
+            out[vo] = x;
+            if (r) r[vo] = wm[vo] * x;
         }
     }
 }
@@ -579,22 +646,19 @@ cudaError_t launch_panel_split_f32(const PanelPiece* pieces, int np, const float
     return cudaGetLastError();
 }
 
-cudaError_t launch_trace_pairs(const TracePair* tp, int n, const double* V, const double* LR, double* part, double* out,
+cudaError_t launch_trace_pairs(const TracePair* tp, int n, const double* V, const double* LR, double* part,
                                cudaStream_t st) {
-    if (!part || !out) return cudaErrorInvalidValue;
-    if (n > 0) {
-        if (!tp || !V || !LR) return cudaErrorInvalidValue;
-        trace_pairs_kernel<<<min(n, 4096), kDotThreads, 0, st>>>(tp, n, V, LR, part);
-    }
-    sum_partial_kernel<<<1, kDotThreads, 0, st>>>(part, n, out);
+    if (n <= 0) return cudaSuccess;
+    if (!tp || !V || !LR || !part) return cudaErrorInvalidValue;
+    trace_pairs_kernel<<<min(n, 4096), kDotThreads, 0, st>>>(tp, n, V, LR, part);
     return cudaGetLastError();
 }
 
 cudaError_t launch_transfer_combine(const CombineBlock* cb, int n, const double* V, const double* T, double* out,
-                                    const double* s, cudaStream_t st) {
+                                    const double* part, int np, const double* wm, double* r, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    if (!cb || !V || !T || !out || !s) return cudaErrorInvalidValue;
-    transfer_combine_kernel<<<min(n, 4096), 256, 0, st>>>(cb, n, V, T, out, s);
+    if (!cb || !V || !T || !out || (np > 0 && !part) || (r && !wm)) return cudaErrorInvalidValue;
+    transfer_combine_kernel<<<dim3(min(n, 4096), n < 152 ? 8 : 1), kDotThreads, 0, st>>>(cb, n, V, T, out, part, np, wm, r);
     return cudaGetLastError();
 }
 
@@ -617,18 +681,20 @@ cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* part
     sum_partial_kernel<<<1, kDotThreads, 0, st>>>(part, nc, out);
     return cudaGetLastError();
 }
-cudaError_t launch_mdot(const double* V, int nv, int64_t n, const double* w, double* part, double* out,
-                        cudaStream_t st) {
-    if (nv <= 0) return cudaSuccess;
+cudaError_t launch_arnoldi_pass(const double* V, int nv, int64_t n, const double* wm, double* w, double* r, double* part,
+                                double* coef, cudaStream_t st) {
+    if (nv < 1 || nv > kArnoldiMax || n <= 0 || !V || !wm || !w || !r || !part || !coef) return cudaErrorInvalidValue;
     const int64_t ch = dot_chunk(n);
     const int nc = dot_nchunk(n);
-    mdot_partial_kernel<<<dim3(nc, nv), kDotThreads, 0, st>>>(V, n, w, ch, nc, part);
-    msum_partial_kernel<<<nv, kDotThreads, 0, st>>>(part, nc, out);
+    arnoldi_dot_kernel<<<dim3(nc, nv), kDotThreads, 0, st>>>(V, n, r, ch, nc, part);
+    if (nc > 32) msum_partial_kernel<<<nv, kDotThreads, 0, st>>>(part, nc, coef);
+    arnoldi_update_kernel<<<grid_for(n, 256, 152 * 8), 256, nv * 8, st>>>(V, nv, n, nc > 32 ? nullptr : part, nc, coef, wm,
+                                                                         w, r);
     return cudaGetLastError();
 }
-cudaError_t launch_mgs(const double* V, int nv, int64_t n, const double* coef, double* w, cudaStream_t st) {
-    if (nv <= 0) return cudaSuccess;
-    mgs_update_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(V, nv, n, coef, w);
+cudaError_t launch_arnoldi_norm(const double* w, const double* r, int64_t n, double* part, double* out, cudaStream_t st) {
+    if (n <= 0 || !w || !r || !part || !out) return cudaErrorInvalidValue;
+    arnoldi_norm_kernel<<<dot_nchunk(n), kDotThreads, 0, st>>>(w, r, n, dot_chunk(n), part, out);
     return cudaGetLastError();
 }
 cudaError_t launch_axpy(double a, const double* x, double* y, int64_t n, cudaStream_t st) {
@@ -641,8 +707,9 @@ cudaError_t launch_hadamard(const double* a, const double* b, double* out, int64
     hadamard_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(a, b, out, n);
     return cudaGetLastError();
 }
-cudaError_t launch_scale(double a, double* x, int64_t n, cudaStream_t st) {
-    scale_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(a, x, n);
+cudaError_t launch_scale(double a, double* x, int64_t n, cudaStream_t st) { return launch_scale_to(a, x, x, n, st); }
+cudaError_t launch_scale_to(double a, const double* x, double* y, int64_t n, cudaStream_t st) {
+    scale_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(a, x, y, n);
     return cudaGetLastError();
 }
 cudaError_t launch_combine(const double* V, int nv, int64_t n, const double* c, double* y, cudaStream_t st) {

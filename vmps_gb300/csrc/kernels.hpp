@@ -97,11 +97,16 @@ cudaError_t launch_pack(const PackBlock* blocks, int nb, const double* src, doub
 int64_t dot_chunk(int64_t n);
 int dot_nchunk(int64_t n);
 cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* part, double* out, cudaStream_t st);
-cudaError_t launch_mdot(const double* V, int nv, int64_t n, const double* w, double* part, double* out,
-                        cudaStream_t st);
-cudaError_t launch_mgs(const double* V, int nv, int64_t n, const double* coef, double* w, cudaStream_t st);
+// One Gram-Schmidt pass of an Arnoldi step on w and r = wm * w: coef[j] = <V_j, r>,
+// w -= sum_j coef[j] V_j, r = wm * w, j < nv.  part holds nv * dot_nchunk(n) doubles.
+constexpr int kArnoldiMax = 1024;
+cudaError_t launch_arnoldi_pass(const double* V, int nv, int64_t n, const double* wm, double* w, double* r, double* part,
+                                double* coef, cudaStream_t st);
+// out[0] = <w, r>; out[4] holds a counter, zero before the first launch
+cudaError_t launch_arnoldi_norm(const double* w, const double* r, int64_t n, double* part, double* out, cudaStream_t st);
 cudaError_t launch_axpy(double a, const double* x, double* y, int64_t n, cudaStream_t st);
 cudaError_t launch_scale(double a, double* x, int64_t n, cudaStream_t st);
+cudaError_t launch_scale_to(double a, const double* x, double* y, int64_t n, cudaStream_t st);   // y = a x
 cudaError_t launch_hadamard(const double* a, const double* b, double* out, int64_t n, cudaStream_t st);   // out = a * b
 cudaError_t launch_combine(const double* V, int nv, int64_t n, const double* c, double* y, cudaStream_t st);
 cudaError_t launch_finite(const double* x, int64_t n, int* bad, cudaStream_t st);
@@ -120,13 +125,14 @@ struct PenaltyArgs {
 };
 cudaError_t launch_penalty(const PenaltyArgs& a, const double* y, const float* yf, double* o, float* of,
                            cudaStream_t st);
-// VUMPS transfer operator: out = sum_b w_b tr(V_b LR_b) (deterministic); out[V block] = V - T + s * 1
+// VUMPS transfer operator: part[b] = w_b tr(V_b LR_b); out[V block] = V - T + (sum_b part[b]) * 1
+// and, r set, r = wm * out there
 struct TracePair { int64_t v_off, lr_off; int32_t rows, cols, v_ld, lr_ld; double weight; };
 struct CombineBlock { int64_t v_off, t_off; int32_t rows, cols, v_ld, t_ld; };
-cudaError_t launch_trace_pairs(const TracePair* tp, int n, const double* V, const double* LR, double* part, double* out,
+cudaError_t launch_trace_pairs(const TracePair* tp, int n, const double* V, const double* LR, double* part,
                                cudaStream_t st);
 cudaError_t launch_transfer_combine(const CombineBlock* cb, int n, const double* V, const double* T, double* out,
-                                    const double* s, cudaStream_t st);
+                                    const double* part, int np, const double* wm, double* r, cudaStream_t st);
 
 // ---- device-resident Lanczos step (lanczos.cu) ----------------------------------
 constexpr int kLzMaxIter = 1024;       // Krylov dimension limit of the device step

@@ -3088,7 +3088,7 @@ struct vmps_transfer_s {
     DevLayout Vd;
     BlockTable LRt;
     DevLayout LRd;
-    DBuf dLR, dVout, stage_in, stage_out, pk, dTrace, dCombine, part, scal;
+    DBuf dLR, dVout, stage_in, stage_out, pk, dTrace, dCombine, part;
     int npk = 0, ntrace = 0, ncombine = 0;
     std::vector<char> prepped[2];
     QN abq;                         // (QN, index) of the slot ab
@@ -3104,19 +3104,20 @@ struct vmps_transfer_s {
 };
 
 // T's operator (VumpsMpoTransferMatrix.h:99-212) on padded device vectors: the cell's
-// contract_L/R chain from din, then Vout = Vin - T Vin + LdotR * 1 on the slot-ab blocks
-static void transfer_apply(vmps_transfer* t, const double* din, double* dout, int prec) {
+// contract_L/R chain from din (each step reads the vector before it where it lies), then
+// Vout = Vin - T Vin + LdotR * 1 on the slot-ab blocks and zero elsewhere; r set: r = wm * Vout
+static void transfer_apply(vmps_transfer* t, const double* din, double* dout, int prec, const double* wm = nullptr,
+                           double* r = nullptr) {
     cudaStream_t st = t->st();
     vmps_env* first = t->chain.front();
-    if (din != first->dE.as<double>() && first->Ed.total > 0)
-        CK(cudaMemcpyAsync(first->dE.p, din, (size_t)first->Ed.total * 8, cudaMemcpyDeviceToDevice, st));
+    const double* y = din;
     for (size_t k = 0; k < t->chain.size(); ++k) {
         vmps_env* e = t->chain[k];
         DevPlan& dp = env_plan(e, prec);
         Operands ops;
         if (e->side == VMPS_ENV_LEFT) { ops.X = e->dB.as<double>(); ops.Z = e->dK.as<double>(); }
         else { ops.X = e->dK.as<double>(); ops.Z = e->dB.as<double>(); }
-        ops.Y = e->dE.as<double>();
+        ops.Y = y;
         ops.O = e->dN.as<double>();
         ops.err = t->ctx->err;
         if (!t->prepped[prec][k]) {   // the site tensors are fixed: their split panels are made once
@@ -3124,14 +3125,13 @@ static void transfer_apply(vmps_transfer* t, const double* din, double* dout, in
             t->prepped[prec][k] = 1;
         }
         run_plan(dp, ops, st);
-        if (k + 1 < t->chain.size() && e->Nd.total > 0)
-            CK(cudaMemcpyAsync(t->chain[k + 1]->dE.p, e->dN.p, (size_t)e->Nd.total * 8, cudaMemcpyDeviceToDevice, st));
+        y = e->dN.as<double>();
     }
-    CK(launch_trace_pairs(t->dTrace.as<TracePair>(), t->ntrace, first->dE.as<double>(), t->dLR.as<double>(),
-                          t->part.as<double>(), t->scal.as<double>(), st));
+    CK(launch_trace_pairs(t->dTrace.as<TracePair>(), t->ntrace, din, t->dLR.as<double>(), t->part.as<double>(), st));
     CK(cudaMemsetAsync(dout, 0, (size_t)std::max<int64_t>(t->Vd.total, 1) * 8, st));
-    CK(launch_transfer_combine(t->dCombine.as<CombineBlock>(), t->ncombine, first->dE.as<double>(),
-                               t->chain.back()->dN.as<double>(), dout, t->scal.as<double>(), st));
+    if (r) CK(cudaMemsetAsync(r, 0, (size_t)std::max<int64_t>(t->Vd.total, 1) * 8, st));
+    CK(launch_transfer_combine(t->dCombine.as<CombineBlock>(), t->ncombine, din, t->chain.back()->dN.as<double>(), dout,
+                               t->part.as<double>(), t->ntrace, wm, r, st));
 }
 
 // ---- device GMRES of the transfer operator --------------------------------------
@@ -3206,7 +3206,7 @@ static int transfer_gmres(vmps_transfer* t, const double* rhs, double* x, double
     const int64_t n = t->Vd.total;
     double* Q = t->gQ.as<double>();
     double* w = t->gw.as<double>();
-    double* r = t->gr.as<double>();
+    double* r = t->gr.as<double>();                  // wm * w
     double* d = t->gd.as<double>();                  // this call's solution
     double* ax = t->dVout.as<double>();
     const double* m = t->gm.as<double>();
@@ -3219,6 +3219,7 @@ static int transfer_gmres(vmps_transfer* t, const double* rhs, double* x, double
     std::vector<double> H((size_t)ld * dimK, 0.0), cs((size_t)dimK), sn((size_t)dimK), g((size_t)ld);
     std::vector<double> col((size_t)(2 * ld + 1));
     CK(cudaMemsetAsync(d, 0, (size_t)n * 8, st));
+    CK(cudaMemsetAsync(hd, 0, (size_t)(2 * ld + 8) * 8, st));
     int its = 0;
     for (int cycle = 0; cycle < max_restarts; ++cycle) {
         // w = mask * (rhs - A d)
@@ -3232,25 +3233,18 @@ static int transfer_gmres(vmps_transfer* t, const double* rhs, double* x, double
         if (!std::isfinite(beta)) throw GmresNonFinite("GMRES: non-finite residual");
         if (beta <= abs_tol) break;
         if (cycle > 0 && restarts) ++*restarts;
-        CK(cudaMemcpyAsync(Q, w, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
-        CK(launch_scale(1.0 / beta, Q, n, st));
+        CK(launch_scale_to(1.0 / beta, w, Q, n, st));
         std::fill(g.begin(), g.end(), 0.0);
         g[0] = beta;
         int kk = 0;
         for (int k = 0; k < dimK; ++k) {
-            transfer_apply(t, Q + (int64_t)k * n, ax, prec);
+            // (zero off the slot-ab blocks: no mask)
+            transfer_apply(t, Q + (int64_t)k * n, w, prec, wm, r);
             ++its;
-            CK(launch_hadamard(m, ax, w, n, st));
-            for (int pass = 0; pass < 2; ++pass) {
-                CK(launch_hadamard(wm, w, r, n, st));
-                CK(launch_mdot(Q, k + 1, n, r, t->gpart.as<double>(), pass ? h2d : hd, st));
-                CK(launch_mgs(Q, k + 1, n, pass ? h2d : hd, w, st));
-            }
-            CK(launch_hadamard(wm, w, r, n, st));
-            CK(launch_dot(w, r, n, t->gpart.as<double>(), nrm, st));
-            CK(cudaMemcpyAsync(col.data(), hd, sizeof(double) * (size_t)(k + 1), cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(col.data() + ld, h2d, sizeof(double) * (size_t)(k + 1), cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(col.data() + 2 * ld, nrm, sizeof(double), cudaMemcpyDeviceToHost, st));
+            CK(launch_arnoldi_pass(Q, k + 1, n, wm, w, r, t->gpart.as<double>(), hd, st));
+            CK(launch_arnoldi_pass(Q, k + 1, n, wm, w, r, t->gpart.as<double>(), h2d, st));
+            CK(launch_arnoldi_norm(w, r, n, t->gpart.as<double>(), nrm, st));
+            CK(cudaMemcpyAsync(col.data(), hd, sizeof(double) * col.size(), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             double* hk = H.data() + (size_t)k * ld;
             for (int j = 0; j <= k; ++j) hk[j] = col[(size_t)j] + col[(size_t)(ld + j)];
@@ -3273,8 +3267,7 @@ static int transfer_gmres(vmps_transfer* t, const double* rhs, double* x, double
             g[(size_t)k] = cs[(size_t)k] * g[(size_t)k];
             kk = k + 1;
             if (hn <= 1e-14 * beta || std::abs(g[(size_t)k + 1]) <= abs_tol || k + 1 == dimK) break;
-            CK(cudaMemcpyAsync(Q + (int64_t)(k + 1) * n, w, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
-            CK(launch_scale(1.0 / hn, Q + (int64_t)(k + 1) * n, n, st));
+            CK(launch_scale_to(1.0 / hn, w, Q + (int64_t)(k + 1) * n, n, st));
         }
         // y = R^-1 g (upper triangular, kk x kk), d += Q y
         std::vector<double> y((size_t)kk, 0.0);
@@ -3409,7 +3402,6 @@ int vmps_transfer_create(vmps_ctx* ctx, const vmps_symmetry* symd, int dir, int 
     upload_vec(t->dTrace, tps, st);
     upload_vec(t->dCombine, cbs, st);
     t->part.alloc((size_t)std::max(1, t->ntrace) * 8, st, true);
-    t->scal.alloc(64, st, true);
     t->dVout.alloc((size_t)std::max<int64_t>(t->Vd.total, 1) * 8, st, true);
     auto pb = pack_blocks(t->Vt, t->Vd, nullptr);
     t->npk = (int)pb.size();
