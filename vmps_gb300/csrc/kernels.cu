@@ -21,6 +21,7 @@
 
 #include "convert.hpp"
 #include "kernels.hpp"
+#include "pdl.cuh"
 
 namespace vmps {
 
@@ -53,9 +54,10 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
     __shared__ double As[2][BK * LD], Bs[2][BK * LD];   // [k][row], [k][column]
     __shared__ GSeg sseg[SEGS];
     __shared__ GTerm sterm[SEGS * kMaxTerms];
+    pdl_wait();
     const GTile tile = g.tiles[blockIdx.x];
-    const double* __restrict__ A = (const double*)g.A + blockIdx.y * g.strideA;
-    const double* __restrict__ B = (const double*)g.B + blockIdx.y * g.strideB;
+    const double* A = pdl_data((const double*)g.A + blockIdx.y * g.strideA);
+    const double* B = pdl_data((const double*)g.B + blockIdx.y * g.strideB);
     const int tid = threadIdx.x, tm = tile.tm, tn = tile.tn, ne = tm * tn;
     const bool tA = g.transA, tB = g.transB;
     // the output elements of this thread, column by column; a second one for tiles of more than 128
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
                                          : (int64_t)(tile.row0 + i) + (int64_t)(k0 + k) * sg.lda;
                     for (int t = 0; t < sg.term_count; ++t) {
                         const GTerm tm_ = sterm[t0 + t];
-                        ra[r] = fma(tm_.coef, __ldg(A + tm_.off + e), ra[r]);
+                        ra[r] = fma(tm_.coef, ld_global(A + tm_.off + e), ra[r]);
                     }
                 }
                 const int j = tB ? lo : hi, kb = tB ? hi : lo;
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
                 if (j < tn && kb < krem) {
                     const int64_t e = tB ? (int64_t)(tile.col0 + j) + (int64_t)(k0 + kb) * sg.ldb
                                          : (int64_t)(k0 + kb) + (int64_t)(tile.col0 + j) * sg.ldb;
-                    rb[r] = __ldg(B + sg.b_off + e);
+                    rb[r] = ld_global(B + sg.b_off + e);
                 }
             }
         };
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
             buf ^= 1;
         }
     }
-    double* __restrict__ C = (double*)g.C + blockIdx.y * g.strideC + tile.c_off;
+    double* C = (double*)g.C + blockIdx.y * g.strideC + tile.c_off;
     auto put = [&](int i, int j, double x) {
         const int64_t gr = tile.row0 + i, gc = tile.col0 + j;
         C[g.transC ? gc + gr * tile.ldc : gr + gc * tile.ldc] = x;
@@ -156,8 +158,9 @@ __device__ __forceinline__ void split_store(__nv_bfloat16* row, int k, float v) 
 }
 
 // operand preparation: scale, split into bf16 hi/lo, write the block's panel rows
-__global__ void prep_kernel(const PrepBlock* __restrict__ pbs, int nb, const double* __restrict__ src,
-                            __nv_bfloat16* __restrict__ dst) {
+__global__ void prep_kernel(const PrepBlock* pbs, int nb, const double* src,
+                            __nv_bfloat16* dst) {
+    pdl_wait();
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
         const PrepBlock pb = pbs[b];
         const int rows = pb.rows, n = pb.rows * pb.cols;
@@ -196,8 +199,9 @@ __device__ __forceinline__ void piece_load4(const double* p, double (&x)[4]) {
     x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 template <typename T>
-__global__ void panel_split_kernel(const PanelPiece* __restrict__ pieces, int np, const T* __restrict__ src,
-                                   __nv_bfloat16* __restrict__ dst) {
+__global__ void panel_split_kernel(const PanelPiece* pieces, int np, const T* src,
+                                   __nv_bfloat16* dst) {
+    pdl_wait();
     for (int b = blockIdx.x; b < np; b += gridDim.x) {
         const PanelPiece pc = pieces[b];
         const int rows = pc.rows, nr4 = (rows + 3) >> 2, ng = nr4 * pc.cols;
@@ -260,8 +264,9 @@ __device__ __forceinline__ void split_store_tf32(float* row, int k, float v) {
     row[p] = h;
     row[p + 16] = to_tf32(v - h);
 }
-__global__ void prep_tf32_kernel(const PrepBlock* __restrict__ pbs, int nb, const double* __restrict__ src,
-                                 float* __restrict__ dst) {
+__global__ void prep_tf32_kernel(const PrepBlock* pbs, int nb, const double* src,
+                                 float* dst) {
+    pdl_wait();
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
         const PrepBlock pb = pbs[b];
         const int rows = pb.rows, n = pb.rows * pb.cols;
@@ -278,8 +283,9 @@ __global__ void prep_tf32_kernel(const PrepBlock* __restrict__ pbs, int nb, cons
 // vector pieces -> 3xTF32 panels: one element per thread (column c of the piece is
 // panel row c, its element r is K index r)
 template <typename T>
-__global__ void panel_split_tf32_kernel(const PanelPiece* __restrict__ pieces, int np, const T* __restrict__ src,
-                                        float* __restrict__ dst) {
+__global__ void panel_split_tf32_kernel(const PanelPiece* pieces, int np, const T* src,
+                                        float* dst) {
+    pdl_wait();
     for (int b = blockIdx.x; b < np; b += gridDim.x) {
         const PanelPiece pc = pieces[b];
         const int rows = pc.rows, n = rows * pc.cols;
@@ -296,8 +302,9 @@ __global__ void panel_split_tf32_kernel(const PanelPiece* __restrict__ pieces, i
 // layout conversion, vector algebra
 // ===========================================================================
 // dst (padded) <- scale * src (compact), or the reverse
-__global__ void pack_kernel(const PackBlock* blocks, int nb, const double* __restrict__ src, double* __restrict__ dst,
+__global__ void pack_kernel(const PackBlock* blocks, int nb, const double* src, double* dst,
                             int to_padded) {
+    pdl_wait();
     for (int b = blockIdx.x; b < nb; b += gridDim.x) {
         const PackBlock pb = blocks[b];
         // pieces hold at most a few thousand elements: 32-bit index arithmetic
@@ -346,8 +353,9 @@ __device__ __forceinline__ double block_tree_sum(double s) {
     }
     return s;
 }
-__global__ void dot_partial_kernel(const double* __restrict__ x, const double* __restrict__ y, int64_t n,
-                                   int64_t chunk, double* __restrict__ part) {
+__global__ void dot_partial_kernel(const double* x, const double* y, int64_t n,
+                                   int64_t chunk, double* part) {
+    pdl_wait();
     const int64_t b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
     double s = 0;
 #pragma unroll 8
@@ -355,7 +363,8 @@ __global__ void dot_partial_kernel(const double* __restrict__ x, const double* _
     s = block_tree_sum(s);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
-__global__ void sum_partial_kernel(const double* __restrict__ part, int np, double* __restrict__ out) {
+__global__ void sum_partial_kernel(const double* part, int np, double* out) {
+    pdl_wait();
     double s = 0;
     for (int i = threadIdx.x; i < np; i += kDotThreads) s += part[i];
     s = block_tree_sum(s);
@@ -370,9 +379,10 @@ __global__ void sum_partial_kernel(const double* __restrict__ part, int np, doub
 // per element and basis row (an operation holds an SM quadrant's pipe for 64 clocks per warp).
 //
 // part[j][chunk] of <V_j, r>, j < nv (V row-major [nv][n])
-__global__ void __launch_bounds__(kDotThreads) arnoldi_dot_kernel(const double* __restrict__ V, int64_t n,
-                                                                  const double* __restrict__ r, int64_t chunk,
-                                                                  int nchunk, double* __restrict__ part) {
+__global__ void __launch_bounds__(kDotThreads) arnoldi_dot_kernel(const double* V, int64_t n,
+                                                                  const double* r, int64_t chunk,
+                                                                  int nchunk, double* part) {
+    pdl_wait();
     const int64_t b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
     const double* v = V + (int64_t)blockIdx.y * n;
     double s = 0;
@@ -382,7 +392,7 @@ __global__ void __launch_bounds__(kDotThreads) arnoldi_dot_kernel(const double* 
     if (threadIdx.x == 0) part[(int64_t)blockIdx.y * nchunk + blockIdx.x] = s;
 }
 // the sum of nchunk <= 32 partials in the order of block_tree_sum (which adds zeros to them)
-__device__ __forceinline__ double partial_tree_sum(const double* __restrict__ p, int nchunk) {
+__device__ __forceinline__ double partial_tree_sum(const double* p, int nchunk) {
     double t[32];
 #pragma unroll
     for (int c = 0; c < 32; ++c) t[c] = c < nchunk ? 0.0 + p[c] : 0.0;
@@ -394,7 +404,8 @@ __device__ __forceinline__ double partial_tree_sum(const double* __restrict__ p,
         }
     return t[0];
 }
-__global__ void msum_partial_kernel(const double* __restrict__ part, int nchunk, double* __restrict__ out) {
+__global__ void msum_partial_kernel(const double* part, int nchunk, double* out) {
+    pdl_wait();
     double s = 0;
     for (int i = threadIdx.x; i < nchunk; i += kDotThreads) s += part[(int64_t)blockIdx.x * nchunk + i];
     s = block_tree_sum(s);
@@ -402,10 +413,11 @@ __global__ void msum_partial_kernel(const double* __restrict__ part, int nchunk,
 }
 // w -= sum_j coef[j] V_j, r = wm * w; part set: coef[j] is summed here from nchunk <= 32 partials by every
 // block, and stored by the first
-__global__ void __launch_bounds__(256) arnoldi_update_kernel(const double* __restrict__ V, int nv, int64_t n,
-                                                             const double* __restrict__ part, int nchunk, double* coef,
-                                                             const double* __restrict__ wm, double* __restrict__ w,
-                                                             double* __restrict__ r) {
+__global__ void __launch_bounds__(256) arnoldi_update_kernel(const double* V, int nv, int64_t n,
+                                                             const double* part, int nchunk, double* coef,
+                                                             const double* wm, double* w,
+                                                             double* r) {
+    pdl_wait();
     extern __shared__ double c[];
     for (int j = threadIdx.x; j < nv; j += blockDim.x) {
         const double x = part ? partial_tree_sum(part + (int64_t)j * nchunk, nchunk) : coef[j];
@@ -423,9 +435,10 @@ __global__ void __launch_bounds__(256) arnoldi_update_kernel(const double* __res
 }
 // out[0] = <w, r>, the partials summed by the last block (out[4]: its counter, zero between
 // launches)
-__global__ void __launch_bounds__(kDotThreads) arnoldi_norm_kernel(const double* __restrict__ w,
-                                                                   const double* __restrict__ r, int64_t n, int64_t chunk,
+__global__ void __launch_bounds__(kDotThreads) arnoldi_norm_kernel(const double* w,
+                                                                   const double* r, int64_t n, int64_t chunk,
                                                                    double* part, double* out) {
+    pdl_wait();
     const int64_t b0 = blockIdx.x * chunk, b1 = min(n, b0 + chunk);
     double s = 0;
 #pragma unroll 16
@@ -449,37 +462,43 @@ __global__ void __launch_bounds__(kDotThreads) arnoldi_norm_kernel(const double*
         *count = 0;
     }
 }
-__global__ void axpy_kernel(double a, const double* __restrict__ x, double* __restrict__ y, int64_t n) {
+__global__ void axpy_kernel(double a, const double* x, double* y, int64_t n) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = fma(a, x[i], y[i]);
 }
-__global__ void hadamard_kernel(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out,
+__global__ void hadamard_kernel(const double* a, const double* b, double* out,
                                 int64_t n) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = a[i] * b[i];
 }
 // y = a x (y = x allowed)
 __global__ void scale_kernel(double a, const double* x, double* y, int64_t n) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = x[i] * a;
 }
 // y = sum_j c[j] V_j  (Ritz vector assembly)
-__global__ void combine_kernel(const double* __restrict__ V, int nv, int64_t n, const double* __restrict__ c,
-                               double* __restrict__ y) {
+__global__ void combine_kernel(const double* V, int nv, int64_t n, const double* c,
+                               double* y) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double s = 0;
         for (int j = 0; j < nv; ++j) s = fma(c[j], V[(int64_t)j * n + i], s);
         y[i] = s;
     }
 }
-__global__ void finite_kernel(const double* __restrict__ x, int64_t n, int* __restrict__ bad) {
+__global__ void finite_kernel(const double* x, int64_t n, int* bad) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         if (!isfinite(x[i])) { atomicOr(bad, 1); return; }
 }
 
 // split-K of the grouped GEMM: out[e] = sum_j part[j * n + e], parts in order
 template <typename T>
-__global__ void splitk_reduce_kernel(const T* __restrict__ part, int nparts, int64_t n, T* __restrict__ out) {
+__global__ void splitk_reduce_kernel(const T* part, int nparts, int64_t n, T* out) {
+    pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double s = (double)part[i];
         for (int j = 1; j < nparts; ++j) s += (double)part[(int64_t)j * n + i];
@@ -495,7 +514,8 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ part, int nparts, int
 // order: the same bits in every run.
 // ---------------------------------------------------------------------------
 template <typename TY>
-__global__ void pen_dot_kernel(PenaltyArgs a, const TY* __restrict__ y) {
+__global__ void pen_dot_kernel(PenaltyArgs a, const TY* y) {
+    pdl_wait();
     __shared__ double red[kDotThreads];
     const int pr = blockIdx.y, p = pr / a.nrhs, r = pr - p * a.nrhs;
     const int64_t b0 = blockIdx.x * a.chunk, b1 = min(a.n, b0 + a.chunk);
@@ -513,6 +533,7 @@ __global__ void pen_dot_kernel(PenaltyArgs a, const TY* __restrict__ y) {
 }
 // coef[p * nrhs + r] = E * (sum of the chunk partials), one block per (p, r)
 __global__ void pen_sum_kernel(PenaltyArgs a) {
+    pdl_wait();
     __shared__ double red[kDotThreads];
     const int pr = blockIdx.x;
     double s = 0;
@@ -526,7 +547,8 @@ __global__ void pen_sum_kernel(PenaltyArgs a) {
     if (threadIdx.x == 0) a.coef[pr] = a.E * red[0];
 }
 template <typename TO>
-__global__ void pen_add_kernel(PenaltyArgs a, TO* __restrict__ out) {
+__global__ void pen_add_kernel(PenaltyArgs a, TO* out) {
+    pdl_wait();
     const int r = blockIdx.y;
     TO* o = out + (int64_t)r * a.n;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -540,9 +562,10 @@ __global__ void pen_add_kernel(PenaltyArgs a, TO* __restrict__ out) {
 // VUMPS transfer operator pieces
 // ---------------------------------------------------------------------------
 // part[b] = w_b * sum_ij V[i + j*v_ld] * LR[j + i*lr_ld]  (the trace of a block product)
-__global__ void __launch_bounds__(kDotThreads) trace_pairs_kernel(const TracePair* __restrict__ tp, int n,
-                                                                  const double* __restrict__ V,
-                                                                  const double* __restrict__ LR, double* __restrict__ part) {
+__global__ void __launch_bounds__(kDotThreads) trace_pairs_kernel(const TracePair* tp, int n,
+                                                                  const double* V,
+                                                                  const double* LR, double* part) {
+    pdl_wait();
     for (int b = blockIdx.x; b < n; b += gridDim.x) {
         const TracePair p = tp[b];
         double s = 0;
@@ -560,13 +583,14 @@ __global__ void __launch_bounds__(kDotThreads) trace_pairs_kernel(const TracePai
 // out[block] = V[block] - T[block] + s * identity, per matched block pair, s the sum of the np trace
 // partials (every block sums them: cheaper than a launch); r set: r = wm * out there as well.
 // gridDim.y blocks share a pair
-__global__ void __launch_bounds__(kDotThreads) transfer_combine_kernel(const CombineBlock* __restrict__ cb, int n,
-                                                                       const double* __restrict__ V,
-                                                                       const double* __restrict__ T,
-                                                                       double* __restrict__ out,
-                                                                       const double* __restrict__ part, int np,
-                                                                       const double* __restrict__ wm,
-                                                                       double* __restrict__ r) {
+__global__ void __launch_bounds__(kDotThreads) transfer_combine_kernel(const CombineBlock* cb, int n,
+                                                                       const double* V,
+                                                                       const double* T,
+                                                                       double* out,
+                                                                       const double* part, int np,
+                                                                       const double* wm,
+                                                                       double* r) {
+    pdl_wait();
     __shared__ double sc_;
     double t = 0;
     for (int i = threadIdx.x; i < np; i += kDotThreads) t += part[i];
@@ -608,41 +632,41 @@ cudaError_t kernels_init() {
 cudaError_t launch_gg64(const GGArgs& a, cudaStream_t st) {
     if (a.ntiles <= 0) return cudaSuccess;
     if (a.nrhs < 1 || a.nrhs > 65535) return cudaErrorInvalidValue;
-    gg_fp64_kernel<<<dim3(a.ntiles, a.nrhs), f64k::NT, 0, st>>>(a);
+    launch_pdl(gg_fp64_kernel, dim3(a.ntiles, a.nrhs), f64k::NT, 0, st, a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_prep(const PrepBlock* pb, int nb, const double* src, void* dst, cudaStream_t st) {
     if (nb <= 0) return cudaSuccess;
     if (!pb || !src || !dst) return cudaErrorInvalidValue;
-    prep_kernel<<<min(nb, 8192), 256, 0, st>>>(pb, nb, src, (__nv_bfloat16*)dst);
+    launch_pdl(prep_kernel, min(nb, 8192), 256, 0, st, pb, nb, src, (__nv_bfloat16*)dst);
     return cudaGetLastError();
 }
 
 cudaError_t launch_panel_split(const PanelPiece* pieces, int np, const double* src, void* dst, cudaStream_t st) {
     if (np <= 0) return cudaSuccess;
     if (!pieces || !src || !dst) return cudaErrorInvalidValue;
-    panel_split_kernel<double><<<min(np, 4096), 256, 0, st>>>(pieces, np, src, (__nv_bfloat16*)dst);
+    launch_pdl(panel_split_kernel<double>, min(np, 4096), 256, 0, st, pieces, np, src, (__nv_bfloat16*)dst);
     return cudaGetLastError();
 }
 cudaError_t launch_prep_tf32(const PrepBlock* pb, int nb, const double* src, void* dst, cudaStream_t st) {
     if (nb <= 0) return cudaSuccess;
     if (!pb || !src || !dst) return cudaErrorInvalidValue;
-    prep_tf32_kernel<<<min(nb, 8192), 256, 0, st>>>(pb, nb, src, (float*)dst);
+    launch_pdl(prep_tf32_kernel, min(nb, 8192), 256, 0, st, pb, nb, src, (float*)dst);
     return cudaGetLastError();
 }
 cudaError_t launch_panel_split_tf32(const PanelPiece* pieces, int np, const double* src, const float* srcf, void* dst,
                                     cudaStream_t st) {
     if (np <= 0) return cudaSuccess;
     if (!pieces || (!src && !srcf) || !dst) return cudaErrorInvalidValue;
-    if (srcf) panel_split_tf32_kernel<float><<<min(np, 4096), 256, 0, st>>>(pieces, np, srcf, (float*)dst);
-    else panel_split_tf32_kernel<double><<<min(np, 4096), 256, 0, st>>>(pieces, np, src, (float*)dst);
+    if (srcf) launch_pdl(panel_split_tf32_kernel<float>, min(np, 4096), 256, 0, st, pieces, np, srcf, (float*)dst);
+    else launch_pdl(panel_split_tf32_kernel<double>, min(np, 4096), 256, 0, st, pieces, np, src, (float*)dst);
     return cudaGetLastError();
 }
 cudaError_t launch_panel_split_f32(const PanelPiece* pieces, int np, const float* src, void* dst, cudaStream_t st) {
     if (np <= 0) return cudaSuccess;
     if (!pieces || !src || !dst) return cudaErrorInvalidValue;
-    panel_split_kernel<float><<<min(np, 4096), 256, 0, st>>>(pieces, np, src, (__nv_bfloat16*)dst);
+    launch_pdl(panel_split_kernel<float>, min(np, 4096), 256, 0, st, pieces, np, src, (__nv_bfloat16*)dst);
     return cudaGetLastError();
 }
 
@@ -650,7 +674,7 @@ cudaError_t launch_trace_pairs(const TracePair* tp, int n, const double* V, cons
                                cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (!tp || !V || !LR || !part) return cudaErrorInvalidValue;
-    trace_pairs_kernel<<<min(n, 4096), kDotThreads, 0, st>>>(tp, n, V, LR, part);
+    launch_pdl(trace_pairs_kernel, min(n, 4096), kDotThreads, 0, st, tp, n, V, LR, part);
     return cudaGetLastError();
 }
 
@@ -658,14 +682,14 @@ cudaError_t launch_transfer_combine(const CombineBlock* cb, int n, const double*
                                     const double* part, int np, const double* wm, double* r, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (!cb || !V || !T || !out || (np > 0 && !part) || (r && !wm)) return cudaErrorInvalidValue;
-    transfer_combine_kernel<<<dim3(min(n, 4096), n < 152 ? 8 : 1), kDotThreads, 0, st>>>(cb, n, V, T, out, part, np, wm, r);
+    launch_pdl(transfer_combine_kernel, dim3(min(n, 4096), n < 152 ? 8 : 1), kDotThreads, 0, st, cb, n, V, T, out, part, np, wm, r);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pack(const PackBlock* blocks, int nb, const double* src, double* dst, int to_padded, cudaStream_t st) {
     if (nb <= 0) return cudaSuccess;
     if (!blocks || !src || !dst) return cudaErrorInvalidValue;   // never launch on an unallocated buffer
-    pack_kernel<<<min(nb, 4096), 256, 0, st>>>(blocks, nb, src, dst, to_padded);
+    launch_pdl(pack_kernel, min(nb, 4096), 256, 0, st, blocks, nb, src, dst, to_padded);
     return cudaGetLastError();
 }
 // chunked dot: part must hold nchunk doubles
@@ -677,8 +701,8 @@ int dot_nchunk(int64_t n) { return (int)((n + dot_chunk(n) - 1) / dot_chunk(n));
 cudaError_t launch_dot(const double* x, const double* y, int64_t n, double* part, double* out, cudaStream_t st) {
     const int64_t ch = dot_chunk(n);
     const int nc = dot_nchunk(n);
-    dot_partial_kernel<<<nc, kDotThreads, 0, st>>>(x, y, n, ch, part);
-    sum_partial_kernel<<<1, kDotThreads, 0, st>>>(part, nc, out);
+    launch_pdl(dot_partial_kernel, nc, kDotThreads, 0, st, x, y, n, ch, part);
+    launch_pdl(sum_partial_kernel, 1, kDotThreads, 0, st, part, nc, out);
     return cudaGetLastError();
 }
 cudaError_t launch_arnoldi_pass(const double* V, int nv, int64_t n, const double* wm, double* w, double* r, double* part,
@@ -686,41 +710,41 @@ cudaError_t launch_arnoldi_pass(const double* V, int nv, int64_t n, const double
     if (nv < 1 || nv > kArnoldiMax || n <= 0 || !V || !wm || !w || !r || !part || !coef) return cudaErrorInvalidValue;
     const int64_t ch = dot_chunk(n);
     const int nc = dot_nchunk(n);
-    arnoldi_dot_kernel<<<dim3(nc, nv), kDotThreads, 0, st>>>(V, n, r, ch, nc, part);
-    if (nc > 32) msum_partial_kernel<<<nv, kDotThreads, 0, st>>>(part, nc, coef);
-    arnoldi_update_kernel<<<grid_for(n, 256, 152 * 8), 256, nv * 8, st>>>(V, nv, n, nc > 32 ? nullptr : part, nc, coef, wm,
+    launch_pdl(arnoldi_dot_kernel, dim3(nc, nv), kDotThreads, 0, st, V, n, r, ch, nc, part);
+    if (nc > 32) launch_pdl(msum_partial_kernel, nv, kDotThreads, 0, st, part, nc, coef);
+    launch_pdl(arnoldi_update_kernel, grid_for(n, 256, 152 * 8), 256, nv * 8, st, V, nv, n, nc > 32 ? nullptr : part, nc, coef, wm,
                                                                          w, r);
     return cudaGetLastError();
 }
 cudaError_t launch_arnoldi_norm(const double* w, const double* r, int64_t n, double* part, double* out, cudaStream_t st) {
     if (n <= 0 || !w || !r || !part || !out) return cudaErrorInvalidValue;
-    arnoldi_norm_kernel<<<dot_nchunk(n), kDotThreads, 0, st>>>(w, r, n, dot_chunk(n), part, out);
+    launch_pdl(arnoldi_norm_kernel, dot_nchunk(n), kDotThreads, 0, st, w, r, n, dot_chunk(n), part, out);
     return cudaGetLastError();
 }
 cudaError_t launch_axpy(double a, const double* x, double* y, int64_t n, cudaStream_t st) {
-    axpy_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(a, x, y, n);
+    launch_pdl(axpy_kernel, grid_for(n, 256, 152 * 8), 256, 0, st, a, x, y, n);
     return cudaGetLastError();
 }
 cudaError_t launch_hadamard(const double* a, const double* b, double* out, int64_t n, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (!a || !b || !out) return cudaErrorInvalidValue;
-    hadamard_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(a, b, out, n);
+    launch_pdl(hadamard_kernel, grid_for(n, 256, 152 * 8), 256, 0, st, a, b, out, n);
     return cudaGetLastError();
 }
 cudaError_t launch_scale(double a, double* x, int64_t n, cudaStream_t st) { return launch_scale_to(a, x, x, n, st); }
 cudaError_t launch_scale_to(double a, const double* x, double* y, int64_t n, cudaStream_t st) {
-    scale_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(a, x, y, n);
+    launch_pdl(scale_kernel, grid_for(n, 256, 152 * 8), 256, 0, st, a, x, y, n);
     return cudaGetLastError();
 }
 cudaError_t launch_combine(const double* V, int nv, int64_t n, const double* c, double* y, cudaStream_t st) {
-    combine_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(V, nv, n, c, y);
+    launch_pdl(combine_kernel, grid_for(n, 256, 152 * 8), 256, 0, st, V, nv, n, c, y);
     return cudaGetLastError();
 }
 cudaError_t launch_splitk_reduce(const void* part, int nparts, int64_t n, void* out, int f32, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (!part || !out || nparts < 1) return cudaErrorInvalidValue;
-    if (f32) splitk_reduce_kernel<float><<<grid_for(n, 256, 152 * 8), 256, 0, st>>>((const float*)part, nparts, n, (float*)out);
-    else splitk_reduce_kernel<double><<<grid_for(n, 256, 152 * 8), 256, 0, st>>>((const double*)part, nparts, n, (double*)out);
+    if (f32) launch_pdl(splitk_reduce_kernel<float>, grid_for(n, 256, 152 * 8), 256, 0, st, (const float*)part, nparts, n, (float*)out);
+    else launch_pdl(splitk_reduce_kernel<double>, grid_for(n, 256, 152 * 8), 256, 0, st, (const double*)part, nparts, n, (double*)out);
     return cudaGetLastError();
 }
 cudaError_t launch_penalty(const PenaltyArgs& a, const double* y, const float* yf, double* o, float* of,
@@ -730,16 +754,16 @@ cudaError_t launch_penalty(const PenaltyArgs& a, const double* y, const float* y
         (int64_t)a.nchunk * a.chunk < a.n)
         return cudaErrorInvalidValue;
     const dim3 gd(a.nchunk, a.npen * a.nrhs);
-    if (yf) pen_dot_kernel<float><<<gd, kDotThreads, 0, st>>>(a, yf);
-    else pen_dot_kernel<double><<<gd, kDotThreads, 0, st>>>(a, y);
-    pen_sum_kernel<<<a.npen * a.nrhs, kDotThreads, 0, st>>>(a);
+    if (yf) launch_pdl(pen_dot_kernel<float>, gd, kDotThreads, 0, st, a, yf);
+    else launch_pdl(pen_dot_kernel<double>, gd, kDotThreads, 0, st, a, y);
+    launch_pdl(pen_sum_kernel, a.npen * a.nrhs, kDotThreads, 0, st, a);
     const dim3 ga(grid_for(a.n, 256, 152 * 4), a.nrhs);
-    if (of) pen_add_kernel<float><<<ga, 256, 0, st>>>(a, of);
-    else pen_add_kernel<double><<<ga, 256, 0, st>>>(a, o);
+    if (of) launch_pdl(pen_add_kernel<float>, ga, 256, 0, st, a, of);
+    else launch_pdl(pen_add_kernel<double>, ga, 256, 0, st, a, o);
     return cudaGetLastError();
 }
 cudaError_t launch_finite(const double* x, int64_t n, int* bad, cudaStream_t st) {
-    finite_kernel<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(x, n, bad);
+    launch_pdl(finite_kernel, grid_for(n, 256, 152 * 8), 256, 0, st, x, n, bad);
     return cudaGetLastError();
 }
 

@@ -38,6 +38,7 @@
 
 #include "convert.hpp"
 #include "kernels.hpp"
+#include "pdl.cuh"
 
 namespace vmps {
 
@@ -179,7 +180,7 @@ __device__ __forceinline__ double lz_block_sums(const V (&v)[R]) {
 // Full chunks go by 16-byte groups where the chunk allows; the partial last chunk element by
 // element.
 template <typename V, int E>
-__device__ __forceinline__ V lz_chunk_dot(const V* __restrict__ ki, const V* wsh, int len, int lane) {
+__device__ __forceinline__ V lz_chunk_dot(const V* ki, const V* wsh, int len, int lane) {
     V s[4] = {0, 0, 0, 0};
     constexpr int W = LzPack<V>::W;
     if (len == E * 256) {
@@ -218,7 +219,7 @@ __device__ __forceinline__ void lz_store_sums(const V (&v)[8], int i0, int m, do
     if ((lane & (32 / R - 1)) == 0 && i < m) part[(int64_t)i * nchunk + blockIdx.x] = t;
 }
 template <typename V, int E>
-__device__ __forceinline__ void lz_all_dots(const V* __restrict__ kb, int64_t ld, int m, const V* wsh, int len,
+__device__ __forceinline__ void lz_all_dots(const V* kb, int64_t ld, int m, const V* wsh, int len,
                                             double* part, int nchunk) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i0 = warp; i0 < m; i0 += 8 * kLzWarps) {
@@ -238,6 +239,7 @@ __device__ __forceinline__ void lz_all_dots(const V* __restrict__ kb, int64_t ld
 
 template <typename V, int E>
 __global__ void __launch_bounds__(kLzThreads) lz_local_kernel(LzArgs a) {
+    pdl_wait();
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
     const int64_t e0 = (int64_t)blockIdx.x * (E * kLzThreads) + threadIdx.x;
@@ -269,6 +271,7 @@ __global__ void __launch_bounds__(kLzThreads) lz_local_kernel(LzArgs a) {
 
 template <typename V, int E>
 __global__ void __launch_bounds__(kLzThreads) lz_proj_kernel(LzArgs a) {
+    pdl_wait();
     __shared__ __align__(16) V wsh[E * kLzThreads];   // this block's chunk of w after the local step
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
@@ -321,6 +324,7 @@ __global__ void __launch_bounds__(kLzThreads) lz_proj_kernel(LzArgs a) {
 
 // d_i = sum over chunks of lz_proj's partials, one block per basis row
 __global__ void __launch_bounds__(kLzThreads) lz_coef_kernel(LzArgs a) {
+    pdl_wait();
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
     for (int i = blockIdx.x; i <= j; i += gridDim.x) {
@@ -331,6 +335,7 @@ __global__ void __launch_bounds__(kLzThreads) lz_coef_kernel(LzArgs a) {
 
 template <typename V, int E>
 __global__ void __launch_bounds__(kLzThreads) lz_orth_kernel(LzArgs a) {
+    pdl_wait();
     const int j = (int)a.ctl[0];
     if (j >= a.kmax) return;
     // the coefficients in the vector type, converted once per block
@@ -429,6 +434,7 @@ __global__ void __launch_bounds__(kLzThreads) lz_orth_kernel(LzArgs a) {
 
 template <typename V>
 __global__ void lz_next_kernel(LzArgs a) {
+    pdl_wait();
     const int jn = (int)a.ctl[0];
     if (jn < 1 || jn > a.kmax) return;
     const V s = (V)a.ab[2 * a.kmax + jn - 1];
@@ -449,8 +455,9 @@ __global__ void lz_next_kernel(LzArgs a) {
 
 // y[e] = sum_{i < m} c[i] K_i[e] in FP64 (Ritz vectors and corrections)
 template <typename V>
-__global__ void lz_combine_kernel(const V* __restrict__ K, int64_t ld, int m, int64_t n,
-                                  const double* __restrict__ c, double* __restrict__ y) {
+__global__ void lz_combine_kernel(const V* K, int64_t ld, int m, int64_t n,
+                                  const double* c, double* y) {
+    pdl_wait();
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
         double s = 0;
         for (int i = 0; i < m; ++i) s = fma(c[i], lz_f64(K[(int64_t)i * ld + e]), s);
@@ -461,9 +468,10 @@ __global__ void lz_combine_kernel(const V* __restrict__ K, int64_t ld, int m, in
 // out[i] = <K_i, r> for i < m, deterministic: per-chunk partials here (r is
 // FP64, rounded to the basis type when staged), summed by lz_rowsum_kernel
 template <typename V, int E>
-__global__ void __launch_bounds__(kLzThreads) lz_mdot_kernel(const V* __restrict__ K, int64_t ld, int m, int64_t n,
-                                                              const double* __restrict__ r,
-                                                              double* __restrict__ part, int nchunk) {
+__global__ void __launch_bounds__(kLzThreads) lz_mdot_kernel(const V* K, int64_t ld, int m, int64_t n,
+                                                              const double* r,
+                                                              double* part, int nchunk) {
+    pdl_wait();
     __shared__ __align__(16) V rsh[E * kLzThreads];
     const int64_t cb = (int64_t)blockIdx.x * (E * kLzThreads);
     const int len = (int)(n - cb < E * kLzThreads ? n - cb : E * kLzThreads);
@@ -479,13 +487,15 @@ __global__ void __launch_bounds__(kLzThreads) lz_mdot_kernel(const V* __restrict
 // out[i] = sum over chunks of part[i], i < rows, one block per row
 __global__ void __launch_bounds__(kLzThreads) lz_rowsum_kernel(const double* part, int nchunk, int rows,
                                                                 double* out) {
+    pdl_wait();
     for (int i = blockIdx.x; i < rows; i += gridDim.x) {
         const double t = lz_block_row_sum(part, i, nchunk);
         if (threadIdx.x == 0) out[i] = t;
     }
 }
 
-__global__ void lz_to_f32_kernel(const double* __restrict__ x, float* __restrict__ y, int64_t n) {
+__global__ void lz_to_f32_kernel(const double* x, float* y, int64_t n) {
+    pdl_wait();
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
         y[e] = f64_to_f32_rn(x[e]);
 }
@@ -500,6 +510,7 @@ __global__ void lz_to_f32_kernel(const double* __restrict__ x, float* __restrict
 // to finish writes the moments and advances n.
 template <int E>
 __global__ void __launch_bounds__(kLzThreads) cheb_step_kernel(ChebArgs a) {
+    pdl_wait();
     const int step = (int)a.ctl[0];
     const double ca = step == 0 ? a.inv_a : 2.0 * a.inv_a, cp = step == 0 ? 0.0 : 1.0;
     const int k = blockIdx.y, pj = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -580,14 +591,14 @@ cudaError_t lz_init() { return cudaSuccess; }
 template <typename V>
 static cudaError_t lz_step(const LzArgs& a, int per_thread, cudaStream_t st) {
 #define LZ_CALL(EE)                                                   \
-    lz_local_kernel<V, EE><<<a.nchunk, kLzThreads, 0, st>>>(a);       \
-    lz_proj_kernel<V, EE><<<a.nchunk, kLzThreads, 0, st>>>(a);        \
-    lz_coef_kernel<<<kLzCoefBlocks, kLzThreads, 0, st>>>(a);           \
-    lz_orth_kernel<V, EE><<<a.nchunk, kLzThreads, 0, st>>>(a);
+    launch_pdl(lz_local_kernel<V, EE>, a.nchunk, kLzThreads, 0, st, a);       \
+    launch_pdl(lz_proj_kernel<V, EE>, a.nchunk, kLzThreads, 0, st, a);        \
+    launch_pdl(lz_coef_kernel, kLzCoefBlocks, kLzThreads, 0, st, a);           \
+    launch_pdl(lz_orth_kernel<V, EE>, a.nchunk, kLzThreads, 0, st, a);
     LZ_DISPATCH(per_thread, LZ_CALL)
 #undef LZ_CALL
     const int g = (int)std::min<int64_t>((a.n + 255) / 256, 152 * 8);
-    lz_next_kernel<V><<<g, 256, 0, st>>>(a);
+    launch_pdl(lz_next_kernel<V>, g, 256, 0, st, a);
     return cudaGetLastError();
 }
 
@@ -603,8 +614,8 @@ cudaError_t launch_lz_combine(const void* K, int fp32, int64_t ld, int m, int64_
                               cudaStream_t st) {
     if (m < 1 || n <= 0 || !K || !c || !y) return cudaErrorInvalidValue;
     const int g = (int)std::min<int64_t>((n + 255) / 256, 152 * 8);
-    if (fp32) lz_combine_kernel<float><<<g, 256, 0, st>>>((const float*)K, ld, m, n, c, y);
-    else lz_combine_kernel<double><<<g, 256, 0, st>>>((const double*)K, ld, m, n, c, y);
+    if (fp32) launch_pdl(lz_combine_kernel<float>, g, 256, 0, st, (const float*)K, ld, m, n, c, y);
+    else launch_pdl(lz_combine_kernel<double>, g, 256, 0, st, (const double*)K, ld, m, n, c, y);
     return cudaGetLastError();
 }
 
@@ -613,13 +624,13 @@ cudaError_t launch_lz_mdot(const void* K, int fp32, int64_t ld, int m, int64_t n
     if (m < 1 || m > kLzMaxIter || n <= 0 || !K || !r || !part || !out) return cudaErrorInvalidValue;
     if ((int64_t)sh.nchunk * sh.chunk < n) return cudaErrorInvalidValue;
 #define LZ_CALL(EE)                                                                                        \
-    if (fp32) lz_mdot_kernel<float, EE><<<sh.nchunk, kLzThreads, 0, st>>>((const float*)K, ld, m, n, r, part, \
+    if (fp32) launch_pdl(lz_mdot_kernel<float, EE>, sh.nchunk, kLzThreads, 0, st, (const float*)K, ld, m, n, r, part, \
                                                                           sh.nchunk);                       \
-    else lz_mdot_kernel<double, EE><<<sh.nchunk, kLzThreads, 0, st>>>((const double*)K, ld, m, n, r, part,   \
+    else launch_pdl(lz_mdot_kernel<double, EE>, sh.nchunk, kLzThreads, 0, st, (const double*)K, ld, m, n, r, part,   \
                                                                         sh.nchunk);
     LZ_DISPATCH(sh.per_thread, LZ_CALL)
 #undef LZ_CALL
-    lz_rowsum_kernel<<<m < kLzCoefBlocks ? m : kLzCoefBlocks, kLzThreads, 0, st>>>(part, sh.nchunk, m, out);
+    launch_pdl(lz_rowsum_kernel, m < kLzCoefBlocks ? m : kLzCoefBlocks, kLzThreads, 0, st, part, sh.nchunk, m, out);
     return cudaGetLastError();
 }
 #undef LZ_DISPATCH
@@ -627,7 +638,7 @@ cudaError_t launch_lz_mdot(const void* K, int fp32, int64_t ld, int m, int64_t n
 cudaError_t launch_lz_to_f32(const double* x, float* y, int64_t n, cudaStream_t st) {
     if (n <= 0 || !x || !y) return cudaErrorInvalidValue;
     const int g = (int)std::min<int64_t>((n + 255) / 256, 152 * 8);
-    lz_to_f32_kernel<<<g, 256, 0, st>>>(x, y, n);
+    launch_pdl(lz_to_f32_kernel, g, 256, 0, st, x, y, n);
     return cudaGetLastError();
 }
 
@@ -640,7 +651,7 @@ cudaError_t launch_cheb_step(const ChebArgs& a, int per_thread, cudaStream_t st)
         if (a.pbeg[j + 1] <= a.pbeg[j] || (int64_t)a.nchunk * per_thread * kLzThreads < a.pbeg[j + 1] - a.pbeg[j])
             return cudaErrorInvalidValue;
     const dim3 grid(a.nchunk, a.nrhs, a.nparts);
-#define LZ_CALL(EE) cheb_step_kernel<EE><<<grid, kLzThreads, 0, st>>>(a);
+#define LZ_CALL(EE) launch_pdl(cheb_step_kernel<EE>, grid, kLzThreads, 0, st, a);
     switch (per_thread) {
         case 1: LZ_CALL(1); break;
         case 2: LZ_CALL(2); break;

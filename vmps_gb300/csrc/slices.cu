@@ -34,6 +34,7 @@
 #include <stdint.h>
 
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace vmps {
@@ -80,7 +81,7 @@ __device__ __forceinline__ void slice_load(const SliceArgs& a, const SliceBlock&
                 const double* p = a.src + tm.off + base + i;
                 double v[UN];
 #pragma unroll
-                for (int u = 0; u < UN; ++u) v[u] = o0 + 4 * u < outer ? __ldg(p + (int64_t)(o0 + 4 * u) * b.ld) : 0.0;
+                for (int u = 0; u < UN; ++u) v[u] = o0 + 4 * u < outer ? p[(int64_t)(o0 + 4 * u) * b.ld] : 0.0;
                 const bool unit = tm.coef == 1.0;
 #pragma unroll
                 for (int u = 0; u < UN; ++u) x[u] = t == 0 ? (unit ? v[u] : tm.coef * v[u]) : fma(tm.coef, v[u], x[u]);
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(sl::NT) slice_kernel(SliceArgs a) {
     using namespace sl;
     extern __shared__ double sh[];
     const int r = threadIdx.x >> 2, g = threadIdx.x & 3;
+    pdl_wait();
     for (int p = blockIdx.x; p < a.npieces; p += gridDim.x) {
         const SlicePiece pc = a.pieces[p];
         const SliceBlock b = a.blocks[pc.block];
@@ -344,9 +346,12 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
         S0 = g.tiles[t0].step0;
         S1 = g.tiles[t1 - 1].step0 + g.tiles[t1 - 1].nsteps;
     }
+    if (tid < 8 && S0 + tid < S1) prefetch_l1(g.steps + S0 + tid);
+    pdl_wait();
 
     if (warp == 0) {
         if (lane == 0) {
+            fence_async_global();
             // stage of step `it` and the parity of its use, counted instead of divided
             int it = 0, st = 0, use = 0;
             SliceStep r{};
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
             return make_int3(r.x, r.y, r.z);
         };
         int3 ge = group(G0), ge1 = group(G0 + 1);
-        int ea = __ldg(g.ea + ge.x + rl), eb = __ldg(g.eb + ge.y + c0 + (lane & 7));
+        int ea = g.ea[ge.x + rl], eb = g.eb[ge.y + c0 + (lane & 7)];
         int grp = 0;
         bool ok = true;
         for (int t = t0; t < t1 && ok; ++t) {
@@ -442,7 +447,7 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
                 for (int c = 0; c < 8; ++c) acc[c] = 0.0;
             }
             for (int q = 0; q < ngroups; ++q, ++grp) {
-                const int ea1 = __ldg(g.ea + ge1.x + rl), eb1 = __ldg(g.eb + ge1.y + c0 + (lane & 7));
+                const int ea1 = g.ea[ge1.x + rl], eb1 = g.eb[ge1.y + c0 + (lane & 7)];
                 const int3 ge2 = group(G0 + grp + 2);
                 const int buf = grp & 1, use = grp >> 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(2 * STAGES + buf), (uint32_t)(use & 1), s_fail, wb));
@@ -562,7 +567,7 @@ cudaError_t launch_slices(const SliceArgs& a, cudaStream_t st) {
     if (!a.pieces || !a.blocks || !a.terms || !a.src || !a.dst || !a.exps || a.kcache < 32 || a.kcache % 32 ||
         a.kcache > kSliceCacheK)
         return cudaErrorInvalidValue;
-    slice_kernel<<<a.npieces < 16384 ? a.npieces : 16384, sl::NT, a.kcache * sl::LD * 8, st>>>(a);
+    launch_pdl(slice_kernel, a.npieces < 16384 ? a.npieces : 16384, sl::NT, a.kcache * sl::LD * 8, st, a);
     return cudaGetLastError();
 }
 
@@ -573,10 +578,10 @@ cudaError_t launch_gg_slices(const SliceGemmArgs& a, const TmaMaps& maps, cudaSt
     if (b.max_arows < 16 || b.max_arows > kSliceTileM) return cudaErrorInvalidValue;
     b.stage_bytes = kSlices * b.max_arows * 64 + sg::B_BYTES;
     b.stages = sg::RING_BYTES / b.stage_bytes < sg::MAX_STAGES ? sg::RING_BYTES / b.stage_bytes : sg::MAX_STAGES;
-    if (b.one_sum && b.one_flush) gg_slice_kernel<true, true><<<b.ncta, sg::NT, sg::SMEM_BYTES, st>>>(b, maps);
-    else if (b.one_sum) gg_slice_kernel<true, false><<<b.ncta, sg::NT, sg::SMEM_BYTES, st>>>(b, maps);
-    else if (!b.one_flush) gg_slice_kernel<false, false><<<b.ncta, sg::NT, sg::SMEM_BYTES, st>>>(b, maps);
-    else gg_slice_kernel<false, true><<<b.ncta, sg::NT, sg::SMEM_BYTES, st>>>(b, maps);
+    if (b.one_sum && b.one_flush) launch_pdl(gg_slice_kernel<true, true>, b.ncta, sg::NT, sg::SMEM_BYTES, st, b, maps);
+    else if (b.one_sum) launch_pdl(gg_slice_kernel<true, false>, b.ncta, sg::NT, sg::SMEM_BYTES, st, b, maps);
+    else if (!b.one_flush) launch_pdl(gg_slice_kernel<false, false>, b.ncta, sg::NT, sg::SMEM_BYTES, st, b, maps);
+    else launch_pdl(gg_slice_kernel<false, true>, b.ncta, sg::NT, sg::SMEM_BYTES, st, b, maps);
     return cudaGetLastError();
 }
 

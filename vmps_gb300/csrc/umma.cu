@@ -23,6 +23,7 @@
 
 #include "convert.hpp"
 #include "kernels.hpp"
+#include "pdl.cuh"
 #include "umma.cuh"
 
 namespace vmps {
@@ -111,19 +112,25 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
     const int t0 = g.cta_tiles[blockIdx.x], t1 = g.cta_tiles[blockIdx.x + 1];
     // main-loop waits give up after wb cycles; the drains before exit keep the full budget
     const long long wb = g.wait_budget > 0 ? g.wait_budget : WAIT_BUDGET;
+    int S0 = 0, S1 = 0;
+    if (warp == 0) {
+        for (int i = lane; i < kMaxMapsA; i += 32) tmap_prefetch(&maps.a[i]);
+        for (int i = lane; i < kMaxMapsB; i += 32) tmap_prefetch(&maps.b[i]);
+        if (t0 < t1) {
+            S0 = g.tiles[t0].step0;
+            S1 = g.tiles[t1 - 1].step0 + g.tiles[t1 - 1].nsteps;
+        }
+        if (lane < 4 && (S0 & ~3) + 4 * lane < S1) prefetch_l1(g.steps + (S0 & ~3) + 4 * lane);
+    } else if (t0 < t1) {
+        prefetch_l1(g.tiles + t0);
+    }
+    pdl_wait();
 
     if (warp == 0) {
         // ---------------- TMA producer: one lane walks the CTA's K steps; their records
         // come through L1, each 128-byte line prefetched 16 steps ahead
-        for (int i = lane; i < kMaxMapsA; i += 32) tmap_prefetch(&maps.a[i]);
-        for (int i = lane; i < kMaxMapsB; i += 32) tmap_prefetch(&maps.b[i]);
         if (lane == 0) {
-            int S0 = 0, S1 = 0;
-            if (t0 < t1) {
-                S0 = g.tiles[t0].step0;
-                S1 = g.tiles[t1 - 1].step0 + g.tiles[t1 - 1].nsteps;
-            }
-            for (int j = S0 & ~3; j < S0 + 16 && j < S1; j += 4) prefetch_l1(g.steps + j);
+            fence_async_global();
             int it = 0;
             for (int j = S0; j < S1; ++j, ++it) {
                 if (((j + 16) & 3) == 0 && j + 16 < S1) prefetch_l1(g.steps + j + 16);
@@ -370,17 +377,17 @@ cudaError_t launch_gg_umma(int out_mode, bool multi, const GGArgs& a, const TmaM
     if (multi && (out_mode == 2 || (out_mode == 0 && a.vstride <= 0))) return cudaErrorInvalidValue;
     if (tf32) {
         if (multi) return cudaErrorInvalidValue;   // 3xTF32 plans have one right-hand side
-        if (out_mode == 1) gg_umma_kernel<1, false, true><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
-        else if (out_mode == 2) gg_umma_kernel<2, false, true><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
-        else if (out_mode == 0) gg_umma_kernel<0, false, true><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
+        if (out_mode == 1) launch_pdl(gg_umma_kernel<1, false, true>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
+        else if (out_mode == 2) launch_pdl(gg_umma_kernel<2, false, true>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
+        else if (out_mode == 0) launch_pdl(gg_umma_kernel<0, false, true>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
         else return cudaErrorInvalidValue;
         return cudaGetLastError();
     }
-    if (out_mode == 1 && !multi) gg_umma_kernel<1, false><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
-    else if (out_mode == 1) gg_umma_kernel<1, true><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
-    else if (out_mode == 2) gg_umma_kernel<2, false><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
-    else if (out_mode == 0 && !multi) gg_umma_kernel<0, false><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
-    else if (out_mode == 0) gg_umma_kernel<0, true><<<a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st>>>(a, maps);
+    if (out_mode == 1 && !multi) launch_pdl(gg_umma_kernel<1, false>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
+    else if (out_mode == 1) launch_pdl(gg_umma_kernel<1, true>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
+    else if (out_mode == 2) launch_pdl(gg_umma_kernel<2, false>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
+    else if (out_mode == 0 && !multi) launch_pdl(gg_umma_kernel<0, false>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
+    else if (out_mode == 0) launch_pdl(gg_umma_kernel<0, true>, a.ncta, um::nt_of(out_mode), um::SMEM_BYTES, st, a, maps);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }

@@ -113,6 +113,8 @@ __device__ __forceinline__ void reg_fence16(uint32_t* r) {
                    "+r"(r[15]));
 }
 
+// writes of earlier kernels, made visible to this thread, before TMA reads of it
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;\n" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];\n" ::"l"(p));
 }
