@@ -16,6 +16,8 @@ struct GGArgs {
     const TStep* steps;
     const int32_t* cta_tiles;
     int ncta;
+    int max_arows, max_brows;               // the phase's largest TMA boxes
+    int stages, a_bytes, stage_bytes;       // of the shared-memory ring (set by launch_gg_umma)
     const GTile* tiles;
     const GSeg* segs;
     const GTerm* terms;

@@ -253,10 +253,15 @@ struct DevPhase {
     DBuf tiles, segs, terms;
     DBuf steps, cta_tiles;   // tcgen05 engine schedule
     std::unique_ptr<TmaMaps> maps;   // tcgen05 engine: the phase's TMA descriptors (kernel parameter)
-    int ntiles = 0, ncta = 0;
+    int ntiles = 0, ncta = 0, max_arows = 16, max_brows = 16;
     const PhasePlan* host = nullptr;
     void upload(const PhasePlan& ph, cudaStream_t st) {
         host = &ph;
+        max_arows = max_brows = 16;
+        for (const TStep& s : ph.steps) {
+            max_arows = std::max(max_arows, (int)s.arows);
+            max_brows = std::max(max_brows, (int)s.brows);
+        }
         ntiles = (int)ph.tiles.size();
         upload_vec(tiles, ph.tiles, st);
         upload_vec(segs, ph.segs, st);
@@ -814,6 +819,8 @@ static void run_phase_on(const DevPlan& dp, int ph, const DevPhase& d, const Pha
     a.steps = d.steps.as<TStep>();
     a.cta_tiles = d.cta_tiles.as<int32_t>();
     a.ncta = d.ncta;
+    a.max_arows = d.max_arows;
+    a.max_brows = d.max_brows;
     a.vstride = dp.plan.vstride;
     if (d.ntiles > 0 && (!a.A || !a.B || !a.C || !a.tiles || !a.steps || !a.cta_tiles || !d.maps))
         throw std::invalid_argument("grouped GEMM launched with an unallocated operand");

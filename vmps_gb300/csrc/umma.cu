@@ -28,19 +28,21 @@
 
 namespace vmps {
 namespace um {
-constexpr int BM = kUmmaTileM, BN = kUmmaTileN, BK = kUmmaBK, STAGES = 4;   // 128 x (<= 256) x 32
+constexpr int BM = kUmmaTileM, BN = kUmmaTileN, BK = kUmmaBK;   // 128 x (<= 256) x 32
 // warp 0 TMA, warp 1 MMA, then the epilogue warps: four for split (panel) outputs, whose
 // staging takes 8 KB of shared memory per warp, eight (two per tensor-memory lane quadrant,
 // alternate 64-column chunks) for FP32 / FP64 outputs
 constexpr int epi_warps(int out_split) { return out_split == 1 ? 4 : 8; }
 constexpr int nt_of(int out_split) { return 64 + 32 * epi_warps(out_split); }
 constexpr int ROW_BYTES = 128;                             // one K step of one row: 32 hi + 32 lo
-constexpr int A_BYTES = BM * ROW_BYTES;                    // A region: 16 KB
-constexpr int B_BYTES = BN * ROW_BYTES;                    // B region, at most: 32 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;             // 48 KB
+// the ring: as many stages of the phase's largest boxes as fit, 4 of 128 + 256 rows (48 KB) to 8.
+// A stage's K step takes 400 to 600 clocks and the way from its products to the next load's
+// arrival ~1,600, so four are just short of covering it.
+constexpr int RING_BYTES = 4 * (BM + BN) * ROW_BYTES, MAX_STAGES = 8;
 constexpr int STAGE_OUT_BYTES = 4 * 8192;                  // split-output epilogue: 32 rows x 256 B per warp
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGE_OUT_BYTES + 1024 + 256;
-static_assert((2 * STAGES + 5) * 8 + 4 * (2 + STAGES) <= 256, "barrier area overflow");
+constexpr int SMEM_BYTES = RING_BYTES + STAGE_OUT_BYTES + 1024 + 256;
+static_assert((2 * MAX_STAGES + 5) * 8 + 8 <= 256, "barrier area overflow");
+static_assert(STAGE_OUT_BYTES >= BM * ROW_BYTES, "the products of a last stage with a low A box read 128 rows");
 constexpr uint32_t ACC_COLS = BN;                          // one FP32 accumulator: 128 lanes x 256 columns
 constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;               // two (all of TMEM), so an epilogue overlaps the next tile
 // kind::tf32: the same with A and B TF32 (format 2 in bits 7-9 and 10-12)
@@ -56,14 +58,11 @@ __device__ __forceinline__ TStep load_step(const TStep* p) {
     s.by = b.x; s.arows = b.y; s.brows = b.z; s.xa = b.w;
     return s;
 }
-__device__ __forceinline__ void tmap_prefetch(const void* tmap) {
-    asm volatile("prefetch.tensormap [%0];\n" ::"l"(tmap) : "memory");
-}
 
 // Persistent, warp-specialised grouped GEMM on panel operands.  CTA b runs
 // tiles[cta_tiles[b] .. cta_tiles[b+1]) (a host-side longest-first schedule),
 // whose K steps are steps[tiles[.].step0 ...], contiguous per CTA.
-//   warp 0, lane 0: per step one TMA box of A and one of B into a 4-deep ring of
+//   warp 0, lane 0: per step one TMA box of A and one of B into a ring of 4 to 8
 //     stages ("full" barriers count the bytes), the step records read through L1
 //     and prefetched ahead;
 //   warp 1 (one lane): per step 2 x (lo*hi, hi*lo, hi*hi) tcgen05.mma into one
@@ -85,11 +84,12 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
     const uint32_t raw = su32(smraw);
     const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;
     const uint32_t ring = raw + pad;   // 1024-aligned: the swizzle pattern is anchored to 1024-byte boundaries
-    unsigned char* stage_out = smraw + pad + STAGES * STAGE_BYTES;
+    const int STAGES = g.stages, A_BYTES = g.a_bytes, STAGE_BYTES = g.stage_bytes;
+    unsigned char* stage_out = smraw + pad + RING_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(stage_out + STAGE_OUT_BYTES);
     // bars[0..S) full, [S..2S) empty, [2S..2S+2) accumulator full, [2S+2..2S+4) accumulator empty,
     // [2S+4] drain of the MMAs issued
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 5);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     auto bar = [&](int i) { return su32(&bars[i]); };
@@ -114,8 +114,6 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
     const long long wb = g.wait_budget > 0 ? g.wait_budget : WAIT_BUDGET;
     int S0 = 0, S1 = 0;
     if (warp == 0) {
-        for (int i = lane; i < kMaxMapsA; i += 32) tmap_prefetch(&maps.a[i]);
-        for (int i = lane; i < kMaxMapsB; i += 32) tmap_prefetch(&maps.b[i]);
         if (t0 < t1) {
             S0 = g.tiles[t0].step0;
             S1 = g.tiles[t1 - 1].step0 + g.tiles[t1 - 1].nsteps;
@@ -131,17 +129,18 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
         // come through L1, each 128-byte line prefetched 16 steps ahead
         if (lane == 0) {
             fence_async_global();
-            int it = 0;
+            // stage of step `it` and the parity of its use, counted instead of divided
+            int it = 0, st = 0, use = 0;
             for (int j = S0; j < S1; ++j, ++it) {
                 if (((j + 16) & 3) == 0 && j + 16 < S1) prefetch_l1(g.steps + j + 16);
                 const TStep r = load_step(g.steps + j);
-                const int st = it % STAGES, use = it / STAGES;
                 if (use >= 1 && !mbar_wait(bar(STAGES + st), (uint32_t)((use - 1) & 1), s_fail, wb)) break;
                 const uint32_t sb = ring + st * STAGE_BYTES;
                 mbar_expect_tx(bar(st), (uint32_t)((r.arows + r.brows) * ROW_BYTES));
                 tma_load_2d(sb, &maps.a[r.amap], r.xa, r.ay, bar(st));
                 // bit 0 of x flags a step whose second K16 slice is padding
                 tma_load_2d(sb + A_BYTES, &maps.b[r.bmap], r.x & ~1, r.by, bar(st));
+                if (++st == STAGES) { st = 0; ++use; }
             }
             // copies still in flight land before the CTA exits (a no-op when the MMA warp consumed them)
             for (int i = it - 1; i >= 0 && i >= it - STAGES; --i)
@@ -149,7 +148,7 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
         }
     } else if (warp == 1 && lane == 0) {
         // ---------------- MMA issuer (the next tile's record is fetched one tile ahead)
-        int it = 0, lt = 0;
+        int st = 0, use = 0, lt = 0;
         GTile tile{};
         if (t0 < t1) tile = g.tiles[t0];
         for (int t = t0; t < t1 && !*s_fail; ++t, ++lt) {
@@ -162,8 +161,7 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
             if (buse >= 1 && !mbar_wait(bar(2 * STAGES + 2 + buf), (uint32_t)((buse - 1) & 1), s_fail, wb)) break;
             tc_fence_after();
             const uint32_t dacc = tmem + (uint32_t)buf * ACC_COLS;
-            for (int k = 0; k < nsteps; ++k, ++it) {
-                const int st = it % STAGES, use = it / STAGES;
+            for (int k = 0; k < nsteps; ++k) {
                 if (!mbar_wait(bar(st), (uint32_t)(use & 1), s_fail, wb)) break;
                 tc_fence_after();
                 const uint32_t sb = ring + st * STAGE_BYTES;
@@ -186,6 +184,7 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
                     }
                 }
                 umma_commit(bar(STAGES + st));
+                if (++st == STAGES) { st = 0; ++use; }
             }
             umma_commit(bar(2 * STAGES + buf));
             tile = next;
@@ -369,8 +368,15 @@ cudaError_t umma_init() {
 
 // multi: the plan's tiles interleave nrhs right-hand sides (separate instances, so
 // that the single-vector epilogues keep their register budget)
-cudaError_t launch_gg_umma(int out_mode, bool multi, const GGArgs& a, const TmaMaps& maps, cudaStream_t st,
+cudaError_t launch_gg_umma(int out_mode, bool multi, const GGArgs& args, const TmaMaps& maps, cudaStream_t st,
                            bool tf32) {
+    GGArgs a = args;
+    if (a.max_arows < 16 || a.max_arows > um::BM || a.max_arows % 16 || a.max_brows < 16 || a.max_brows > um::BN ||
+        a.max_brows % 16)
+        return cudaErrorInvalidValue;
+    a.a_bytes = a.max_arows * um::ROW_BYTES;
+    a.stage_bytes = a.a_bytes + a.max_brows * um::ROW_BYTES;
+    a.stages = um::RING_BYTES / a.stage_bytes < um::MAX_STAGES ? um::RING_BYTES / a.stage_bytes : um::MAX_STAGES;
     if (a.ntiles <= 0) return cudaSuccess;
     if (!a.steps || !a.cta_tiles || a.ncta <= 0 || !a.C) return cudaErrorInvalidValue;
     if (out_mode == 1 && !a.transC) return cudaErrorInvalidValue;   // the staged epilogue writes panel rows
