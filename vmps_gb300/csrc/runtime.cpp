@@ -223,7 +223,10 @@ struct vmps_ctx_s {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // host<->device transfers overlapped with compute
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-    int* err = nullptr;   // device error word written by the tcgen05 engine
+    // error word written by the tcgen05 engines, in mapped host memory: the kernels touch it only to
+    // report, and the host reads it after each call without a copy and a second wait for it
+    int* err_host = nullptr;
+    int* err = nullptr;   // the device's address of it
     bool pageable_access = false;   // the device reads pageable host memory in place
     int num_sms = 152;              // CTAs of the persistent tcgen05 engine (host-only: GB300's count)
     long long wait_budget = 0;      // main-loop wait budget of the tcgen05 engine in cycles (0: ~2 s)
@@ -232,12 +235,11 @@ struct vmps_ctx_s {
 
 // read and clear the device error word (after the stream has been synchronised)
 static void check_device_error(vmps_ctx* c) {
-    if (!c || !c->err) return;
-    int h = 0;
-    CK(cudaMemcpyAsync(&h, c->err, 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    if (!c || !c->err_host) return;
+    volatile int* word = c->err_host;
+    const int h = *word;
     if (h) {
-        CK(cudaMemsetAsync(c->err, 0, 4, c->stream));
+        *word = 0;
         throw WaitTimeout("a bounded device wait in the tcgen05 engine ran out (error word " + std::to_string(h) + ")");
     }
 }
@@ -1470,8 +1472,9 @@ int vmps_ctx_create(int device, vmps_ctx** out) {
     CK(cudaEventCreate(&c->ev0));
     CK(cudaEventCreate(&c->ev1));
     CK(cudaEventCreate(&c->ev2));
-    CK(cudaMalloc((void**)&c->err, 64));
-    CK(cudaMemset(c->err, 0, 64));
+    CK(cudaHostAlloc((void**)&c->err_host, 64, cudaHostAllocMapped));
+    std::memset(c->err_host, 0, 64);
+    CK(cudaHostGetDevicePointer((void**)&c->err, c->err_host, 0));
     int pma = 0, pmt = 0;
     if (cudaDeviceGetAttribute(&pma, cudaDevAttrPageableMemoryAccess, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&pmt, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device) != cudaSuccess) {
@@ -1499,7 +1502,7 @@ int vmps_ctx_destroy(vmps_ctx* ctx) {
     cudaEventDestroy(ctx->ev0);
     cudaEventDestroy(ctx->ev1);
     cudaEventDestroy(ctx->ev2);
-    if (ctx->err) cudaFree(ctx->err);
+    if (ctx->err_host) cudaFreeHost(ctx->err_host);
     cudaStreamSynchronize(ctx->copy_stream);
     // the context's own workspaces go while its stream lives
     ctx->lz.reset();

@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
         }
     }
     __syncthreads();
-    if (*s_fail && tid == 0 && g.err) atomicOr(g.err, 1);
+    if (*s_fail && tid == 0 && g.err) atomicOr_system(g.err, 1);   // (mapped host memory)
     tc_fence_after();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
 }

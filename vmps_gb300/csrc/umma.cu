@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(um::nt_of(OUT_SPLIT), 1)
         }
     }
     __syncthreads();
-    if (*s_fail && tid == 0 && g.err) atomicOr(g.err, 1);
+    if (*s_fail && tid == 0 && g.err) atomicOr_system(g.err, 1);   // (mapped host memory)
     tc_fence_after();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
 }
