@@ -87,7 +87,11 @@ __global__ void __launch_bounds__(f64k::NT) gg_fp64_kernel(GGArgs g) {
                 if (i < tm && k < krem) {
                     const int64_t e = tA ? (int64_t)(k0 + k) + (int64_t)(tile.row0 + i) * sg.lda
                                          : (int64_t)(tile.row0 + i) + (int64_t)(k0 + k) * sg.lda;
-                    for (int t = 0; t < sg.term_count; ++t) {
+                    // a first term of coefficient 1 (every segment of phase 1) takes no FP64 operation
+                    const GTerm first = sterm[t0];
+                    const double x = ld_global(A + first.off + e);
+                    ra[r] = __double_as_longlong(first.coef) == 0x3ff0000000000000ll ? x : fma(first.coef, x, 0.0);
+                    for (int t = 1; t < sg.term_count; ++t) {
                         const GTerm tm_ = sterm[t0 + t];
                         ra[r] = fma(tm_.coef, ld_global(A + tm_.off + e), ra[r]);
                     }
