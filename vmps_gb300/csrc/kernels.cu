@@ -33,7 +33,7 @@ namespace vmps {
 // instruction feeds it (an 8x8x4 DMMA holds its quadrant for 512 clocks), so DMMA
 // has no rate to gain and loses what its fragments round up: the blocks of these
 // tensors are 5 to 200 wide.  64 x 64 DMMA tiles left an 11 x 11 block to one
-// warp of one SM (72 us per launch at D = 64, now ~15); here the elements of a
+// warp of one SM (72 us per launch at D = 64, now ~11); here the elements of a
 // tile spread over all four quadrants without rounding, and the tiles over more
 // SMs.  Large blocks gain as well: whole D = 1024 and 4096 two-site HxVs went from
 // 0.76 to 0.43 ms and from 17.9 to 16.3 ms, the FP64 pipe bounding both.  Small

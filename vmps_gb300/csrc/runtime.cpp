@@ -2405,8 +2405,9 @@ constexpr double kRoundMinRatio = 10;
 
 // The ratio comes from a cost model of the plans (not from timings, so that the
 // choice, and with it every result bit, does not depend on the run): GEMM work at
-// the rates the engines reach on GB300 (FP64 DMMA 0.87 TFLOP/s, bf16 tensor work
-// as issued 530 TFLOP/s), the Lanczos step's vector reads and writes at 5 TB/s,
+// fixed rates (FP64 0.87 TFLOP/s, bf16 tensor work as issued 530 TFLOP/s; the exact
+// slices of large FP64 plans run faster, but a changed rate would change which
+// solves refine by rounds, and with it their results), the Lanczos step's vector reads and writes at 5 TB/s,
 // and 3 us per launch.
 constexpr double kFp64FlopsPerMs = 0.87e9, kTensorFlopsPerMs = 5.3e11, kStepBytesPerMs = 5.0e9,
                  kLaunchMs = 0.003;

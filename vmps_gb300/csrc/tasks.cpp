@@ -1138,15 +1138,15 @@ int32_t slice_box_a(int32_t tm, bool fine) {
 //
 // FMAs run at ~0.75 TFLOP/s (1.35 us per MFLOP).  A slice tile costs ~2.7 us of one of 152
 // SMs whatever its size (0.018 us), the slices ~0.3 us per MFLOP more, and the plan two
-// launches (~8 us) more.  Whole HxVs, FMAs against slices: two-site Hubbard 141 / 158 us at
-// 55 MFLOP and 4,000 tiles, 222 / 186 at 130; one-site Hubbard 83 / 89 at 13 MFLOP, 155 / 109
-// at 68; two-site Heisenberg 87 / 80 at 7, 160 / 103 at 55; SU(2)xU(1) cylinder 109 / 113 at
-// 10, 152 / 124 at 25.
+// launches (~4 us) more.  Whole HxVs, FMAs against slices: two-site Hubbard 122 / 135 us at
+// 55 MFLOP and 4,000 tiles, 206 / 162 at 130; one-site Hubbard 65 / 67 at 13 MFLOP, 139 / 87
+// at 68; two-site Heisenberg 55 / 58 at 7, 138 / 80 at 55; SU(2)xU(1) cylinder 90 / 92 at
+// 10, 132 / 101 at 25.
 //
 // A plan that is applied once (an environment update) would pay for the slices of all three
 // operands and for a longer list of steps: FMAs.  Whole updates, FMAs against slices: Hubbard
-// 1252 / 1291 us at 68 MFLOP, 2296 / 1999 at 500, 7654 / 3762 at 4,000; cylinder 1874 / 2155 at
-// 48, 2623 / 2554 at 280.  It is a small part of a sweep, whose split-precision HxVs round the
+// 1182 / 1252 us at 68 MFLOP, 2263 / 1945 at 500, 7703 / 3724 at 4,000; cylinder 1846 / 2105 at
+// 48, 2598 / 2483 at 280.  It is a small part of a sweep, whose split-precision HxVs round the
 // environment to FP32, so it keeps its order of summation at every size.
 bool slice_engine(double flops, double tiles, bool once) {
     const char* v = std::getenv("VMPS_FP64_ENGINE");
