@@ -64,8 +64,8 @@ constexpr uint64_t kDigitBias = 256ull * ((1ull << 54) + (1ull << 45) + (1ull <<
                                           (1ull << 9) + 1ull);
 
 // values of up to 32 panel rows and K indices [k0, k0 + kn) into shared memory; the lanes of a
-// warp run along the contiguous dimension.  A first term with coefficient 1 takes no FP64
-// operation, a further one takes one.
+// warp run along the contiguous dimension.  A first term with coefficient 1 or -1 takes
+// no FP64 operation (nor does the look at it), a further one takes one.
 __device__ __forceinline__ void slice_load(const SliceArgs& a, const SliceBlock& b, int row0, int rows, int k0, int kn,
                                            double* sh) {
     using namespace sl;
@@ -82,9 +82,14 @@ __device__ __forceinline__ void slice_load(const SliceArgs& a, const SliceBlock&
                 double v[UN];
 #pragma unroll
                 for (int u = 0; u < UN; ++u) v[u] = o0 + 4 * u < outer ? p[(int64_t)(o0 + 4 * u) * b.ld] : 0.0;
-                const bool unit = tm.coef == 1.0;
+                const int64_t cb = __double_as_longlong(tm.coef), sign = cb & INT64_MIN;
+                if (t == 0 && (cb ^ sign) == 0x3ff0000000000000ll) {
 #pragma unroll
-                for (int u = 0; u < UN; ++u) x[u] = t == 0 ? (unit ? v[u] : tm.coef * v[u]) : fma(tm.coef, v[u], x[u]);
+                    for (int u = 0; u < UN; ++u) x[u] = __longlong_as_double(__double_as_longlong(v[u]) ^ sign);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < UN; ++u) x[u] = t == 0 ? tm.coef * v[u] : fma(tm.coef, v[u], x[u]);
+                }
             }
 #pragma unroll
             for (int u = 0; u < UN; ++u)
