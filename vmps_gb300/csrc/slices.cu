@@ -459,6 +459,10 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
                 if (!ok) break;
                 tc_fence_after();
                 const bool end = ONE_FLUSH || (ge.z & kSliceSumEnd);
+                // an exponent the integer conversion has no room for, or a bad row or column: each row's is
+                // known to its own lane, each column's to four lanes, whether or not those have a row
+                const bool far = __any_sync(0xffffffffu, (rows && (unsigned)(ea + 440) > 880u) ||
+                                                             (c0 + (lane & 7) < tn && (unsigned)(eb + 440) > 880u));
                 if (cols) {
 #pragma unroll
                     for (int h = 0; h < 8; h += W) {
@@ -495,7 +499,7 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
                             if (!end) continue;
                             const int64_t ldc = ONE_SUM ? tile.ldc : 0;
                             double* C = ONE_SUM ? g.C + tile.c_off + tile.row0 + rl + (tile.col0 + c0) * ldc : nullptr;
-                            rare = (unsigned)(ea + 440) > 880u || (unsigned)(eb + 440) > 880u;
+                            rare = 0;
                             double y[P];
 #pragma unroll
                             for (int c = 0; c < P; ++c) {
@@ -504,7 +508,7 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
                                 const int64_t p = slice_pack(z, e);
                                 y[c] = ONE_SUM || (h + i + c) % 4 == 3 ? slice_to_double_cvt(p, e) : slice_to_double(p, e, rare);
                             }
-                            if (__any_sync(0xffffffffu, rows && rare)) {
+                            if (far || __any_sync(0xffffffffu, rows && rare)) {
 #pragma unroll
                                 for (int c = 0; c < P; ++c) {
                                     const SliceSum z = ONE_FLUSH ? x[c] : part[h + i + c];
