@@ -47,10 +47,14 @@ extern "C" {
 
 /* ---- arithmetic of the block products --------------------------------------*/
 #define VMPS_PREC_FP64       0   /* FP64, parity with the Eigen path: FP64 FMAs, or for large plans
-                                    the tensor cores on an error-free splitting of the operands, whose
-                                    error is no larger (a row or column with an Inf or NaN gives NaN);
-                                    the environment variable VMPS_FP64_ENGINE = auto | fma | slices
-                                    pins the choice                                            */
+                                    the tensor cores on a splitting of the operands into bf16 slices.
+                                    The error bound of a block product's entry is that of FMAs for
+                                    the largest sum of |a b| in its column (products with L) or row
+                                    (with R), in any scaling of the bonds: entries far below the
+                                    others there are less precise than by FMAs.  A row or column with
+                                    an Inf or NaN gives NaN.  The environment variable
+                                    VMPS_FP64_ENGINE = auto | fma | slices pins the choice (fma:
+                                    every entry to the precision of its own sum)               */
 #define VMPS_PREC_BF16X3     1   /* hi*hi + hi*lo + lo*hi bf16 products, FP32 accumulate */
 #define VMPS_PREC_TF32X3     2   /* the same three products with TF32 hi/lo operands (3xTF32): about
                                     2^-21 relative per product against 2^-16, at half the bf16 tensor

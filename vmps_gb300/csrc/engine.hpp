@@ -3,6 +3,7 @@
 #pragma once
 #include <array>
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -213,8 +214,8 @@ struct PhasePlan {
 
 // ---------------------------------------------------------------------------
 // FP64 plans on the tensor cores (slices.cu): operands as panels of seven base-512
-// digit slices in bf16 with one exponent per panel row.  Element (row i, K index k)
-// of slice s is at off + i*pitch + (k/32)*224 + s*32 + k%32, pitch = 7*kpad.
+// digit slices in bf16 with one exponent per panel row, and one per K index of each block of X and Z.
+// Element (row i, K index k) of slice s is at off + i*pitch + (k/32)*224 + s*32 + k%32, pitch = 7*kpad.
 // ---------------------------------------------------------------------------
 constexpr int kSlices = 7;
 constexpr int kSliceTileM = 128, kSliceTileN = 32;
@@ -222,17 +223,20 @@ constexpr int kSliceK = 32;          // K extent of one step
 constexpr int kSliceFlushK = 64;     // K columns an FP32 accumulator sums exactly
 constexpr int kSliceSumK = 192;      // K columns whose flushes a 64-bit integer sums exactly
 constexpr int kSliceBad = 1 << 20;   // exponent of a row that holds an Inf or NaN
+constexpr int kSliceNone = -(1 << 24);   // exponent of a K index at which a block of X or Z is zero
 // one block to slice: panel row i is source row i (trans 1) or source column i (trans 0)
-// of the sum of the terms' blocks (same leading dimension)
-struct SliceBlock { int64_t dst_off; int32_t erow, rows, K, pitch, trans, ld, term_begin, term_count; };
-struct SlicePiece { int32_t block, row0; };   // 32 panel rows of a block
+// of the sum of the terms' blocks (same leading dimension).  koff: the block's exponents along K, for
+// a block of Y or S those of the block of X or Z it is multiplied with
+struct SliceBlock { int64_t dst_off; int32_t erow, rows, K, pitch, trans, ld, term_begin, term_count, koff; };
+struct SlicePiece { int32_t block, row0; };   // 32 panel rows of a block (of kpieces: 32 K indices)
 struct SliceOperand {
     PanelArena arena;
     std::vector<OpBlock> op;          // off, outer (rows), K, cls, row, pitch; pad = first exponent row
     std::vector<SliceBlock> blocks;
     std::vector<GTerm> terms;
-    std::vector<SlicePiece> pieces;
+    std::vector<SlicePiece> pieces, kpieces;
     int64_t rows = 0;                 // exponents
+    int64_t ks = 0;                   // exponents along K (X, Z)
 };
 // one K step: descriptors, slice coordinates (7 * K / 32) and panel rows of the A and B boxes
 struct SliceStep { int32_t amap, bmap, az, bz, ay, by, arows, flags; };
@@ -305,10 +309,13 @@ struct SplitTiling {
     int ncap1 = 256, ncap2 = 256, splitk = 1;
     bool operator==(const SplitTiling& o) const { return ncap1 == o.ncap1 && ncap2 == o.ncap2 && splitk == o.splitk; }
 };
+// The exponents along K of a slice operand's blocks (koff, ks), from their data: make_plan asks for
+// those of the operand that meets Y
+using SliceColumns = std::function<std::vector<int32_t>(const SliceOperand&, bool z)>;
 // FP64 plan: two phases, the second sums first-stage products on the fly; once: applied a single
 // time, so that the slices of X and Z are made for it alone
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z,
-               const DevLayout& O, bool transX, bool transZ, bool once = false);
+               const DevLayout& O, bool transX, bool transZ, bool once = false, const SliceColumns& columns = nullptr);
 // Split-precision plan for the tcgen05 engine: op(X), Y and the chain-scaled
 // copies c*op(Z) in panels; phase 1 computes the intermediates T = op(X)Y into
 // panels, phase 2 the outputs as K-concatenations over chains.

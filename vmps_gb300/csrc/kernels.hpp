@@ -65,6 +65,7 @@ cudaError_t launch_prep_tf32(const PrepBlock* pb, int nb, const double* src, voi
 cudaError_t launch_panel_split_tf32(const PanelPiece* pieces, int np, const double* src, const float* srcf, void* dst,
                                     cudaStream_t st);
 // FP64 on the tensor cores (slices.cu): operand slices, and the grouped GEMM on them
+// (launch_slice_columns: the exponents along K of X or Z, before their slices)
 struct SliceArgs {
     const SlicePiece* pieces;
     const SliceBlock* blocks;
@@ -72,6 +73,8 @@ struct SliceArgs {
     const double* src;
     void* dst;        // digit panels
     int32_t* exps;    // row exponents
+    int32_t* kexp;    // exponents along K, taken from the elements (ksign -1: X, Z) or added to them (1: Y, S)
+    int ksign;
     int npieces;
     int kcache;       // K indices of 32 rows kept in shared memory: a multiple of 32 up to kSliceCacheK
 };
@@ -92,6 +95,7 @@ struct SliceGemmArgs {
     long long wait_budget;
 };
 cudaError_t slices_init();
+cudaError_t launch_slice_columns(const SliceArgs& a, cudaStream_t st);
 cudaError_t launch_slices(const SliceArgs& a, cudaStream_t st);
 cudaError_t launch_gg_slices(const SliceGemmArgs& a, const TmaMaps& maps, cudaStream_t st);
 cudaError_t launch_pack(const PackBlock* blocks, int nb, const double* src, double* dst, int to_padded,

@@ -278,18 +278,34 @@ struct DevPhase {
 
 // device copies of one operand's slice lists and panels, and of one slice phase
 struct DevSliceOperand {
-    DBuf blocks, terms, pieces, panels, exps;
-    int npieces = 0, kcache = 32;
+    DBuf blocks, terms, pieces, kpieces, panels, exps, kexp;
+    int npieces = 0, nkpieces = 0, kcache = 32;
     void upload(const SliceOperand& s, cudaStream_t st) {
         npieces = (int)s.pieces.size();
         for (const SliceBlock& b : s.blocks) kcache = std::max(kcache, std::min(kSliceCacheK, (b.K + 31) / 32 * 32));
         upload_vec(blocks, s.blocks, st);
         upload_vec(terms, s.terms, st);
         upload_vec(pieces, s.pieces, st);
+        nkpieces = (int)s.kpieces.size();
+        upload_vec(kpieces, s.kpieces, st);
+        kexp.alloc((size_t)std::max<int64_t>(s.ks, 1) * 4, st, true);
         panels.alloc((size_t)s.arena.total * 2, st, true);   // zero-filled: panel padding stays zero
         exps.alloc((size_t)(s.rows + 128) * 4, st, true);       // (the flush reads whole tiles' worth)
     }
-    void run(const double* src, cudaStream_t st) const {
+    // X, Z: their own exponents along K, then their slices
+    void prepare(const double* src, cudaStream_t st) const {
+        SliceArgs a{};
+        a.pieces = kpieces.as<SlicePiece>();
+        a.blocks = blocks.as<SliceBlock>();
+        a.terms = terms.as<GTerm>();
+        a.src = src;
+        a.kexp = kexp.as<int32_t>();
+        a.npieces = nkpieces;
+        CK(launch_slice_columns(a, st));
+        run(src, kexp, -1, st);
+    }
+    // Y, S: slices relative to the exponents along K of X or Z
+    void run(const double* src, const DBuf& ke, int ksign, cudaStream_t st) const {
         SliceArgs a{};
         a.pieces = pieces.as<SlicePiece>();
         a.blocks = blocks.as<SliceBlock>();
@@ -297,11 +313,34 @@ struct DevSliceOperand {
         a.src = src;
         a.dst = panels.p;
         a.exps = exps.as<int32_t>();
+        a.kexp = ke.as<int32_t>();
+        a.ksign = ksign;
         a.npieces = npieces;
         a.kcache = kcache;
         CK(launch_slices(a, st));
     }
 };
+// the exponents along K of an operand's blocks, on the host
+static std::vector<int32_t> slice_columns(const SliceOperand& F, const double* src, cudaStream_t st) {
+    std::vector<int32_t> e((size_t)F.ks);
+    if (F.ks == 0) return e;
+    DBuf blocks, terms, kpieces, kexp;
+    upload_vec(blocks, F.blocks, st);
+    upload_vec(terms, F.terms, st);
+    upload_vec(kpieces, F.kpieces, st);
+    kexp.alloc(e.size() * 4, st, false);
+    SliceArgs a{};
+    a.pieces = kpieces.as<SlicePiece>();
+    a.blocks = blocks.as<SliceBlock>();
+    a.terms = terms.as<GTerm>();
+    a.src = src;
+    a.kexp = kexp.as<int32_t>();
+    a.npieces = (int)F.kpieces.size();
+    CK(launch_slice_columns(a, st));
+    CK(cudaMemcpyAsync(e.data(), kexp.p, e.size() * 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return e;
+}
 struct DevSlicePhase {
     DBuf tiles, steps, groups, cta_tiles;
     std::unique_ptr<TmaMaps> maps;
@@ -761,8 +800,8 @@ static void plan_to_device(DevPlan& dp, const DevLayout& Y, cudaStream_t st) {
 // split plans: the bf16 panels of the X and scaled Z operands; slice plans: their slices
 static void split_prepare(DevPlan& dp, const double* X, const double* Z, cudaStream_t st) {
     if (dp.plan.slices) {
-        dp.sx.run(X, st);
-        dp.sz.run(Z, st);
+        dp.sx.prepare(X, st);
+        dp.sz.prepare(Z, st);
         return;
     }
     if (!dp.plan.split) return;
@@ -837,7 +876,7 @@ static void run_phase(const DevPlan& dp, int ph, const Operands& ops, cudaStream
         if (ph == 1) {
             dp.s1.run(xy ? dp.sx : dp.sy, xy ? dp.sy : dp.sz, T, ops.err, ops.wait_budget, st);
         } else {
-            dp.ss.run(T, st);   // the sums of first-stage products, sliced
+            dp.ss.run(T, xy ? dp.sz.kexp : dp.sx.kexp, 1, st);   // the sums of first-stage products, sliced
             dp.s2.run(xy ? dp.ss : dp.sx, xy ? dp.sz : dp.ss, ops.O, ops.err, ops.wait_budget, st);
         }
         return;
@@ -849,7 +888,7 @@ static void run_phase(const DevPlan& dp, int ph, const Operands& ops, cudaStream
 // one application of a planned contraction: (split plans) split Y, phase 1, phase 2
 static void run_plan(const DevPlan& dp, const Operands& ops, cudaStream_t st) {
     if ((ops.Yf || ops.Of) && !dp.plan.split) throw std::invalid_argument("FP32 vectors need a split plan");
-    if (dp.plan.slices) dp.sy.run(ops.Y, st);
+    if (dp.plan.slices) dp.sy.run(ops.Y, dp.plan.association == 0 ? dp.sx.kexp : dp.sz.kexp, 1, st);
     if (dp.plan.split && dp.plan.elt == 4) {
         CK(launch_panel_split_tf32(dp.ypieces.as<PanelPiece>(), dp.nypieces, ops.Yf ? nullptr : ops.Y, ops.Yf, dp.Y2.p,
                                    st));
@@ -1015,7 +1054,12 @@ static DevPlan& get_plan(vmps_pivot* p, int prec) {
     DevPlan& dp = p->plans[prec];
     if (dp.ready) return dp;
     if (prec == VMPS_PREC_FP64) {
-        dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false);
+        SliceColumns columns;
+        if (p->ctx->device >= 0)
+            columns = [&](const SliceOperand& F, bool z) {
+                return slice_columns(F, (z ? p->dR : p->dL).as<double>(), p->st());
+            };
+        dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, false, columns);
         schedule_and_validate(dp.plan, p->ctx->num_sms);
     } else if (prec == VMPS_PREC_TF32X3) {
         dp.plan = make_split_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, 1, SplitTiling(), true);

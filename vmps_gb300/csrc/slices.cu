@@ -1,18 +1,31 @@
-// FP64 grouped GEMM on the tensor cores by exact slices (sm_103a).
+// FP64 grouped GEMM on the tensor cores by slices (sm_103a).
 //
 // GB300's FP64 pipe does two FMAs per clock and SM; tcgen05 does 4096 bf16 ones.
-// An error-free splitting (the scheme of Ozaki, Ogita, Oishi and Rump, 2012)
-// turns an FP64 product into bf16 products that lose nothing: with E the
-// exponent of a panel row's largest element, every element is rounded to an
-// integer multiple of 2^(E-61) and written as seven signed base-512 digits,
+// A splitting (the scheme of Ozaki, Ogita, Oishi and Rump, 2012) turns an FP64
+// product into sums of bf16 products without rounding: with E the exponent of a
+// panel row's largest element, every element is rounded to an integer multiple
+// of 2^(E-61) and written as seven signed base-512 digits,
 //     x = 2^(E-7) sum_s d_s 512^-s,   |d_0| <= 128, -256 <= d_s <= 255,
-// and each digit is a bf16 value exactly.  The sum over K <= 64 of the products of
+// and each digit is a bf16 value exactly.  Elements more than 2^8 below their row's largest lose
+// bits that way, so rows are levelled first: one factor of each product, F (L or R, which do not change), is scaled
+// along K by powers of two to columns of one magnitude, and the other, V, by their inverses.
+// After that no element of V is rounded against one that F would make small.
+//
+// Error of sum_k F_ik V_kj, with M_j the largest over i of sum_k |F_ik V_kj|: the scaled row maxima multiply to
+// at most 4 M_j; rounding the elements costs K 2^-61 of it, the dropped orders (below) K 2^-58.4: K 2^-56
+// M_j in all, where FMAs are bounded by K 2^-53 sum_k |F_ik V_kj|.  Exponents along K are shared by blocks
+// alike within 3 bits (tasks.cpp), which makes it K 2^-53 M_j at most.  So an entry's error is that of FMAs
+// for the largest sum of its column (products with L; with R: of its row), whatever the grading of the
+// contracted index, of the rows and of the columns; an entry far below the others there is less precise than by
+// FMAs.
+//
+// The sum over K <= 64 of the products of
 // equal order d = i + j,
 //     S_d = sum_{i+j=d} sum_k a_i(k) b_j(k),   |S_d| <= 2^24 for d <= 4,
 // is an integer an FP32 accumulator holds exactly (a rounding of S_5 or S_6, which
 // only digits all near their largest could cause, is below 2^-58 of the row and
 // column maxima); orders d <= 6 are kept, 28 of the 49 slice pairs, and the dropped
-// ones lie below 2^-61 each.  An accumulator is flushed after at most 64 columns of
+// products lie below 2^-61 each.  An accumulator is flushed after at most 64 columns of
 // K: the multiple of 2^(Ea+Eb-63) nearest to 2^(Ea+Eb-14) sum_d S_d 512^-d is formed
 // in integers (fine enough for products with identity-like blocks, whose results lie
 // far below the row and column maxima times K); up to three flushes (192 columns) of one
@@ -20,6 +33,7 @@
 // rounding errors left are two per 64 to 192 columns, against one per product by FMAs.
 // Rows with an Inf or NaN give NaN.
 //
+// slice_columns  : the exponents along K of L's and R's blocks, when a plan is made
 // slice_kernel   : FP64 blocks (or sums of blocks) -> digit panels and row exponents
 // gg_slice_kernel: the grouped GEMM on digit panels, FP64 output
 //
@@ -48,20 +62,30 @@ constexpr int LD = ROWS + 1;         // values of K index k at k * LD
 constexpr int UN = 8;                // loads a thread keeps in flight per term
 }
 
-// x as a signed multiple of 2^(E-61), E = emax - 1022 (emax: the row's largest
-// exponent field, at least 1), rounded to nearest
-__device__ __forceinline__ int64_t slice_fixed(double x, int emax) {
+// x 2^s as a signed multiple of 2^(E-61), E = emax - 1022 (emax: the row's largest
+// exponent field after the scaling), rounded to nearest; NORMAL: x is a normal number
+template <bool NORMAL>
+__device__ __forceinline__ int64_t slice_fixed(double x, int s, int emax) {
     const uint64_t bits = (uint64_t)__double_as_longlong(x);
     const int ef = (int)(bits >> 52) & 0x7ff;
-    const uint64_t m = (bits & 0xfffffffffffffull) | (ef ? 1ull << 52 : 0ull);
-    const int sh = emax - max(ef, 1);
-    uint64_t q = m << 8;
-    if (sh > 0) q = sh < 63 ? (q + (1ull << (sh - 1))) >> sh : 0ull;
+    uint64_t q = (bits & 0xfffffffffffffull) << 8;
+    if (NORMAL || ef) q |= 1ull << 60;
+    const int sh = min(emax - s - (NORMAL ? ef : max(ef, 1)), 63);
+    if (NORMAL || sh >= 0) q = (q + ((1ull << sh) >> 1)) >> sh;
+    else if (q) q <<= -sh;   // (a subnormal row maximum)
     return (bits >> 63) ? -(int64_t)q : (int64_t)q;
 }
 // 256 in every base-512 digit: digit s of q is field s of q + kDigitBias, less 256
 constexpr uint64_t kDigitBias = 256ull * ((1ull << 54) + (1ull << 45) + (1ull << 36) + (1ull << 27) + (1ull << 18) +
                                           (1ull << 9) + 1ull);
+
+// the exponent field x has or, subnormal, would have; kSliceNone for zero, 0x7ff for Inf and NaN
+__device__ __forceinline__ int slice_field(double x) {
+    const int f = (__double2hiint(x) >> 20) & 0x7ff;
+    if (f) return f;
+    const uint64_t m = (uint64_t)__double_as_longlong(x) & 0xfffffffffffffull;
+    return m ? 12 - __clzll((long long)m) : kSliceNone;
+}
 
 // values of up to 32 panel rows and K indices [k0, k0 + kn) into shared memory; the lanes of a
 // warp run along the contiguous dimension.  A first term with coefficient 1 or -1 takes
@@ -97,12 +121,16 @@ __device__ __forceinline__ void slice_load(const SliceArgs& a, const SliceBlock&
         }
 }
 
-// digits of eight consecutive K indices of a row: one 16-byte store per slice
-__device__ __forceinline__ void slice_store8(__nv_bfloat16* o, const double* x, int left, int emax, bool bad) {
+// digits of eight consecutive K indices of a row (zero where sk is kSliceNone or the row is bad): one
+// 16-byte store per slice
+template <bool NORMAL>
+__device__ __forceinline__ void slice_store8(__nv_bfloat16* o, const double* x, const int* sk, int emax) {
+    const int4 s0 = reinterpret_cast<const int4*>(sk)[0], s1 = reinterpret_cast<const int4*>(sk)[1];
+    const int s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
     uint64_t q8[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q)
-        q8[q] = (uint64_t)slice_fixed(q < left && !bad ? x[q * sl::LD] : 0.0, emax) + kDigitBias;
+        q8[q] = (uint64_t)slice_fixed<NORMAL>(x[q * sl::LD], s[q], emax) + kDigitBias;
 #pragma unroll
     for (int s = 0; s < kSlices; ++s) {
         uint32_t w[4];
@@ -117,15 +145,63 @@ __device__ __forceinline__ void slice_store8(__nv_bfloat16* o, const double* x, 
     }
 }
 
+// Exponents along K of the blocks of X or Z: 2^e <= |largest finite element at K index k| < 2^(e+1).  Read
+// once when a plan's fixed operands are prepared: bound by memory.
+__global__ void __launch_bounds__(sl::NT) slice_columns_kernel(SliceArgs a) {
+    using namespace sl;
+    __shared__ int red[NT / 32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto field = [](double x) {
+        const int f = slice_field(x);
+        return f == 0x7ff ? kSliceNone : f;
+    };
+    pdl_wait();
+    for (int p = blockIdx.x; p < a.npieces; p += gridDim.x) {
+        const SlicePiece pc = a.pieces[p];
+        const SliceBlock b = a.blocks[pc.block];
+        const int k0 = pc.row0, kn = min(32, b.K - k0);
+        const double* src = a.src + a.terms[b.term_begin].off;
+        if (b.trans) {   // panel rows are contiguous: a warp takes every fourth K index
+            for (int k = warp; k < kn; k += NT / 32) {
+                int f = kSliceNone;
+#pragma unroll 8
+                for (int i = lane; i < b.rows; i += 32) f = max(f, field(src[i + (int64_t)(k0 + k) * b.ld]));
+                f = __reduce_max_sync(0xffffffffu, f);
+                if (lane == 0) red[0][k] = f;
+            }
+        } else {         // K indices are: a warp takes every fourth panel row
+            int f = kSliceNone;
+            if (lane < kn)
+#pragma unroll 8
+                for (int i = warp; i < b.rows; i += NT / 32) f = max(f, field(src[k0 + lane + (int64_t)i * b.ld]));
+            red[warp][lane] = f;
+        }
+        __syncthreads();
+        if (warp == 0 && lane < kn) {
+            int f = red[0][lane];
+            if (!b.trans)
+#pragma unroll
+                for (int w = 1; w < NT / 32; ++w) f = max(f, red[w][lane]);
+            a.kexp[b.koff + k0 + lane] = f == kSliceNone ? kSliceNone : f - 1023;
+        }
+        __syncthreads();
+    }
+}
+
 // Bound by memory for large blocks (8 bytes read per term, 14 written per element)
 // and by latency for small ones.  The sums of the terms go through shared memory,
 // loaded along the contiguous dimension of the block whichever way it lies; then
 // four threads share a panel row and take its octets of K in turn.  The digits
-// come from integer shifts: in FP64 arithmetic they would cost 21 operations per element on the slow pipe.  Rows longer than the shared buffer
-// (a.kcache) are loaded twice, once for the exponent and once for the digits.
-__global__ void __launch_bounds__(sl::NT) slice_kernel(SliceArgs a) {
+// come from integer shifts: in FP64 arithmetic they would cost 21 operations per element on the slow pipe.
+// Rows of normal numbers alone take a form without the tests for the others.  Rows longer than the shared
+// buffer (a.kcache) are loaded twice, once for the exponent and once for the digits.  Scalings along K add an
+// addition and a shared-memory load per element and pass: 31.5 -> 32.3 us for the sums of the D = 1024 two-site
+// Hubbard HxV (37.8 us while the last octet of a row had a form of its own, which warps then ran besides the other).
+__global__ void __launch_bounds__(sl::NT, 6) slice_kernel(SliceArgs a) {
     using namespace sl;
     extern __shared__ double sh[];
+    int* sk = reinterpret_cast<int*>(sh + a.kcache * LD);   // the chunk's exponents along K, as scalings
+    constexpr int EMPTY = -(1 << 25), BAD = 1 << 25;
     const int r = threadIdx.x >> 2, g = threadIdx.x & 3;
     pdl_wait();
     for (int p = blockIdx.x; p < a.npieces; p += gridDim.x) {
@@ -134,33 +210,56 @@ __global__ void __launch_bounds__(sl::NT) slice_kernel(SliceArgs a) {
         const int rows = min(ROWS, b.rows - pc.row0), row = pc.row0 + r;
         const bool on = r < rows;
         __nv_bfloat16* d = (__nv_bfloat16*)a.dst + b.dst_off + (int64_t)row * b.pitch;
-        int emax = 1;
-        bool bad = false;
+        int emax = EMPTY;
+        bool bad = false, normal = true, odd = false;   // odd: the thread met a zero, subnormal number, Inf or NaN
+        auto row_max = [&] {
+            emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 1));
+            emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 2));
+            bad = emax >= BAD / 2;                 // Inf or NaN: digits of zero, the row's products become NaN
+            normal = !__any_sync(0xffffffffu, odd);
+            if (emax < kSliceNone / 2) emax = 1022;   // nothing but zeros, or opposite zeros of the other operand
+        };
         const int passes = b.K <= a.kcache ? 1 : 2;
         for (int pass = 0; pass < passes; ++pass) {
             for (int k0 = 0; k0 < b.K; k0 += a.kcache) {
                 const int kn = min(a.kcache, b.K - k0);
                 __syncthreads();   // the buffer is free
+                // (loaded before the elements, stored after them: one wait for both)
+                static_assert(kSliceCacheK == 2 * NT, "two exponents along K per thread");
+                const int t0 = threadIdx.x, t1 = t0 + NT;
+                const int e0 = t0 < kn ? a.kexp[b.koff + k0 + t0] : 0, e1 = t1 < kn ? a.kexp[b.koff + k0 + t1] : 0;
                 slice_load(a, b, pc.row0, rows, k0, kn, sh);
+                if (t0 < a.kcache) sk[t0] = t0 < kn ? a.ksign * e0 : kSliceNone;   // (past the row's end: zero digits)
+                if (t1 < a.kcache) sk[t1] = t1 < kn ? a.ksign * e1 : kSliceNone;
                 __syncthreads();
-                if (pass == 0 && on)
-                    for (int k = g; k < kn; k += 4) emax = max(emax, (__double2hiint(sh[k * LD + r]) >> 20) & 0x7ff);
-                if (pass + 1 == passes) {
-                    if (passes == 1) {
-                        emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 1));
-                        emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 2));
-                        bad = emax == 0x7ff;   // Inf or NaN: the row's products become NaN
+                if (pass == 0 && on) {
+                    int e = emax;
+                    bool again = false;
+                    for (int k = g; k < kn; k += 4) {
+                        const int f = (__double2hiint(sh[k * LD + r]) >> 20) & 0x7ff;
+                        again |= (unsigned)(f - 1) >= 0x7feu;
+                        e = max(e, f + sk[k]);
                     }
+                    odd |= again;
+                    if (again)
+                        for (int k = g; k < kn; k += 4) {
+                            const int f = slice_field(sh[k * LD + r]);
+                            emax = max(emax, f == 0x7ff ? BAD : f == kSliceNone ? EMPTY : f + sk[k]);
+                        }
+                    else
+                        emax = e;
+                }
+                if (pass + 1 == passes) {
+                    if (passes == 1) row_max();
                     if (on)
-                        for (int k = g * 8; k < kn; k += 32)
-                            slice_store8(d + ((k0 + k) >> 5) * (kSlices * kSliceK) + ((k0 + k) & 31), sh + k * LD + r, kn - k, emax, bad);
+                        for (int k = g * 8; k < kn; k += 32) {
+                            __nv_bfloat16* o = d + ((k0 + k) >> 5) * (kSlices * kSliceK) + ((k0 + k) & 31);
+                            if (normal) slice_store8<true>(o, sh + k * LD + r, sk + k, emax);
+                            else slice_store8<false>(o, sh + k * LD + r, sk + k, emax);
+                        }
                 }
             }
-            if (pass == 0 && passes == 2) {
-                emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 1));
-                emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, 2));
-                bad = emax == 0x7ff;
-            }
+            if (pass == 0 && passes == 2) row_max();
         }
         if (on && g == 0) a.exps[b.erow + row] = bad ? kSliceBad : emax - 1022;
     }
@@ -561,7 +660,7 @@ __global__ void __launch_bounds__(sg::NT, 1) gg_slice_kernel(const SliceGemmArgs
 
 cudaError_t slices_init() {
     const cudaError_t e = cudaFuncSetAttribute(slice_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kSliceCacheK * sl::LD * 8);
+                                               kSliceCacheK * (sl::LD * 8 + 4));
     if (e != cudaSuccess) return e;
     auto opt = [](auto* k) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sg::SMEM_BYTES); };
     cudaError_t r;
@@ -571,12 +670,19 @@ cudaError_t slices_init() {
     return opt(gg_slice_kernel<false, false>);
 }
 
+cudaError_t launch_slice_columns(const SliceArgs& a, cudaStream_t st) {
+    if (a.npieces <= 0) return cudaSuccess;
+    if (!a.pieces || !a.blocks || !a.terms || !a.src || !a.kexp) return cudaErrorInvalidValue;
+    launch_pdl(slice_columns_kernel, a.npieces < 16384 ? a.npieces : 16384, sl::NT, 0, st, a);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_slices(const SliceArgs& a, cudaStream_t st) {
     if (a.npieces <= 0) return cudaSuccess;
-    if (!a.pieces || !a.blocks || !a.terms || !a.src || !a.dst || !a.exps || a.kcache < 32 || a.kcache % 32 ||
-        a.kcache > kSliceCacheK)
+    if (!a.pieces || !a.blocks || !a.terms || !a.src || !a.dst || !a.exps || !a.kexp || (a.ksign != 1 && a.ksign != -1) ||
+        a.kcache < 32 || a.kcache % 32 || a.kcache > kSliceCacheK)
         return cudaErrorInvalidValue;
-    launch_pdl(slice_kernel, a.npieces < 16384 ? a.npieces : 16384, sl::NT, a.kcache * sl::LD * 8, st, a);
+    launch_pdl(slice_kernel, a.npieces < 16384 ? a.npieces : 16384, sl::NT, a.kcache * (sl::LD * 8 + 4), st, a);
     return cudaGetLastError();
 }
 

@@ -12,6 +12,7 @@
 // the W value folded into a single scalar.  The planner then merges duplicate
 // chains, shares first-stage products and lays the work out as tile lists.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -1070,8 +1071,10 @@ PhasePlan make_product_plan(const DevLayout& A, const DevLayout& B, const DevLay
 // FP64 slice engine (slices.cu)
 // ===========================================================================
 namespace {
-// a block of `outer` panel rows of contraction length K; trans and ld as in SliceBlock
-int32_t add_slice_block(SliceOperand& s, int64_t outer, int64_t K, int trans, int64_t ld, const GTerm* terms, size_t n) {
+// a block of `outer` panel rows of contraction length K; trans and ld as in SliceBlock; koff: of
+// the block it is multiplied with, or -1 for a block with exponents along K of its own
+int32_t add_slice_block(SliceOperand& s, int64_t outer, int64_t K, int trans, int64_t ld, const GTerm* terms, size_t n,
+                        int32_t koff) {
     const int32_t kp = panel_kpad(K);
     size_t c = 0;
     while (c < s.arena.cls.size() && s.arena.cls[c].kpad != kp) ++c;
@@ -1095,6 +1098,12 @@ int32_t add_slice_block(SliceOperand& s, int64_t outer, int64_t K, int trans, in
     sb.term_count = (int32_t)n;
     s.terms.insert(s.terms.end(), terms, terms + n);
     const int32_t id = (int32_t)s.op.size();
+    sb.koff = koff;
+    if (koff < 0) {
+        sb.koff = (int32_t)s.ks;
+        s.ks += K;
+        for (int32_t k = 0; k < b.K; k += 32) s.kpieces.push_back(SlicePiece{id, k});
+    }
     for (int32_t r = 0; r < b.outer; r += 32) s.pieces.push_back(SlicePiece{id, r});
     s.rows += outer;
     s.op.push_back(b);
@@ -1113,6 +1122,55 @@ void finish_slices(SliceOperand& s) {
         s.op[i].off = s.arena.cls[s.op[i].cls].base + (int64_t)s.op[i].row * s.op[i].pitch;
         s.blocks[i].dst_off = s.op[i].off;
     }
+}
+// Blocks of F (X or Z) that meet the same blocks of Y share exponents along K, and so the slices
+// of Y, where theirs differ by a constant but for kSliceSpread: `e` are the exponents of the blocks' data, meets
+// the (block of F, block of Y) pairs of the first phase.  Each bit of spread doubles the bound of a
+// product's error (slices.cu); 3 leave it at the FMAs', K 2^-53.  A block that is zero at other K indices does not
+// share: an element of Y that it does not see could be the largest of its column there.  Two-site Hubbard HxVs at
+// D = 1024 / 4096: 201 us / 2.10 ms; with slices of Y for each block 228 / 2.39, a spread of 2 205 / 2.16, of 8
+// 200 / 2.10.
+constexpr int kSliceSpread = 3;
+void share_slice_columns(SliceOperand& F, const std::vector<int32_t>& e, const std::vector<std::pair<int32_t, int64_t>>& meets,
+                         int64_t ny) {
+    std::vector<int32_t> root(F.op.size());
+    std::iota(root.begin(), root.end(), 0);
+    auto find = [&](int32_t x) {
+        while (root[x] != x) x = root[x] = root[root[x]];
+        return x;
+    };
+    std::vector<int32_t> first((size_t)ny, -1);
+    for (const auto& m : meets) {
+        if (first[m.second] < 0) first[m.second] = m.first;
+        const int32_t a = find(first[m.second]), b = find(m.first);
+        root[std::max(a, b)] = std::min(a, b);
+    }
+    auto alike = [&](const SliceBlock& a, const SliceBlock& b) {
+        int lo = INT_MAX, hi = INT_MIN;
+        for (int32_t k = 0; k < a.K; ++k) {
+            const int32_t ea = e[(size_t)a.koff + k], eb = e[(size_t)b.koff + k];
+            if ((ea == kSliceNone) != (eb == kSliceNone)) return false;
+            if (ea == kSliceNone) continue;
+            lo = std::min(lo, ea - eb);
+            hi = std::max(hi, ea - eb);
+            if (hi - lo > kSliceSpread) return false;
+        }
+        return true;
+    };
+    std::vector<std::vector<int32_t>> own(F.op.size());   // per connected set: the blocks with exponents of their own
+    std::vector<char> shares(F.op.size(), 0);
+    for (size_t x = 0; x < F.op.size(); ++x) {
+        std::vector<int32_t>& set = own[find((int32_t)x)];
+        for (int32_t y : set)
+            if (F.blocks[x].K == F.blocks[y].K && alike(F.blocks[x], F.blocks[y])) {
+                F.blocks[x].koff = F.blocks[y].koff;
+                shares[x] = 1;
+                break;
+            }
+        if (!shares[x]) set.push_back((int32_t)x);
+    }
+    F.kpieces.erase(std::remove_if(F.kpieces.begin(), F.kpieces.end(), [&](const SlicePiece& p) { return shares[p.block]; }),
+                    F.kpieces.end());
 }
 void add_slice_tiles(SlicePhase& ph, int64_t c_off, int64_t ldc, int64_t m, int64_t n, int32_t sb, int32_t se) {
     for (const auto& rs : split_extent(m, 1, kSliceTileM))
@@ -1284,6 +1342,7 @@ void validate_slices(const SlicePhase& ph, const SliceOperand& A, const SliceOpe
         for (int32_t s = ph.tile_segs[i][0]; s < ph.tile_segs[i][1]; ++s) {
             const OpBlock &a = A.op.at(ph.segs.at(s).a), &b = B.op.at(ph.segs[s].b);
             need(a.K == b.K && a.K > 0 && t.row0 + t.tm <= a.outer && t.col0 + t.tn <= b.outer, "tile outside its operands");
+            need(A.blocks[ph.segs[s].a].koff == B.blocks[ph.segs[s].b].koff, "factors scaled apart along K");
         }
         bool open = false;
         int ngroups = 0, k = 0;
@@ -1321,7 +1380,7 @@ void validate_slices(const SlicePhase& ph, const SliceOperand& A, const SliceOpe
 }
 
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z, const DevLayout& O,
-               bool transX, bool transZ, bool once) {
+               bool transX, bool transZ, bool once, const SliceColumns& columns) {
     Plan P;
     // shapes: op(X) m x k, Y k x n, op(Z) n x p, out m x p
     auto xm = [&](int64_t x) { return transX ? X.cols[x] : X.rows[x]; };
@@ -1427,29 +1486,46 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
     }
     p1.slotC = SLOT_T;
     p1.transC = false;
-    // slice engine: the operand blocks in use, made on first use
-    std::vector<int32_t> ix(X.rows.size(), -1), iy(Y.rows.size(), -1), iz(Z.rows.size(), -1);
+    // slice engine: the operand blocks in use, made on first use; a block of Y once for all blocks of X or Z
+    // it meets that share exponents along K, relative to which its slices are
+    std::vector<int32_t> ix(X.rows.size(), -1), iz(Z.rows.size(), -1);
     auto slice_x = [&](int64_t x) {
         const GTerm t{X.off[x], 1.0};
-        if (ix[x] < 0) ix[x] = add_slice_block(P.sx, xm(x), xk(x), transX ? 0 : 1, X.ld[x], &t, 1);
+        if (ix[x] < 0) ix[x] = add_slice_block(P.sx, xm(x), xk(x), transX ? 0 : 1, X.ld[x], &t, 1, -1);
         return ix[x];
     };
     auto slice_z = [&](int64_t z) {
         const GTerm t{Z.off[z], 1.0};
-        if (iz[z] < 0) iz[z] = add_slice_block(P.sz, zp(z), zn(z), transZ ? 1 : 0, Z.ld[z], &t, 1);
+        if (iz[z] < 0) iz[z] = add_slice_block(P.sz, zp(z), zn(z), transZ ? 1 : 0, Z.ld[z], &t, 1, -1);
         return iz[z];
     };
-    auto slice_y = [&](int64_t y) {   // columns of Y (association 0: B operand) or its rows (1: A operand)
+    KeyIndex ykeys(P.slices ? ipairs.size() : 0);
+    auto slice_y = [&](int64_t y, int32_t koff) {   // columns of Y (association 0: B operand) or its rows (1: A operand)
+        const auto r = ykeys.add(Key4{y, koff, 0, 0});
+        if (!r.second) return (int32_t)r.first;
         const GTerm t{Y.off[y], 1.0};
         const bool cols = P.association == 0;
-        if (iy[y] < 0)
-            iy[y] = add_slice_block(P.sy, cols ? Y.cols[y] : Y.rows[y], cols ? Y.rows[y] : Y.cols[y], cols ? 0 : 1, Y.ld[y], &t, 1);
-        return iy[y];
+        return add_slice_block(P.sy, cols ? Y.cols[y] : Y.rows[y], cols ? Y.rows[y] : Y.cols[y], cols ? 0 : 1, Y.ld[y], &t, 1,
+                               koff);
     };
+    if (P.slices && columns) {
+        std::vector<std::pair<int32_t, int64_t>> meets;
+        for (const auto& q : ipairs)
+            meets.push_back(P.association == 0 ? std::make_pair(slice_x(q.first), q.second)
+                                               : std::make_pair(slice_z(q.second), q.first));
+        SliceOperand& F = P.association == 0 ? P.sx : P.sz;
+        share_slice_columns(F, columns(F, P.association != 0), meets, (int64_t)Y.rows.size());
+    }
     for (size_t j = 0; P.slices && j < ipairs.size(); ++j) {
         const int64_t a = ipairs[j].first, b = ipairs[j].second;
         const int32_t sb = (int32_t)P.s1.segs.size();
-        P.s1.segs.push_back(P.association == 0 ? SliceSeg{slice_x(a), slice_y(b)} : SliceSeg{slice_y(a), slice_z(b)});
+        if (P.association == 0) {
+            const int32_t x = slice_x(a);
+            P.s1.segs.push_back(SliceSeg{x, slice_y(b, P.sx.blocks[x].koff)});
+        } else {
+            const int32_t z = slice_z(b);
+            P.s1.segs.push_back(SliceSeg{slice_y(a, P.sz.blocks[z].koff), z});
+        }
         p1.flops += 2.0 * trows[j] * tcols[j] * (P.association == 0 ? xk(a) : Y.cols[a]);
         add_slice_tiles(P.s1, P.T.off[j], P.T.ld[j], trows[j], tcols[j], sb, sb + 1);
     }
@@ -1532,10 +1608,13 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
                 // S, the sum of the terms: A operand (rows of T) or B operand (columns of U)
                 const GTerm* tt = p2.terms.data() + s.term_begin;
                 const size_t nt = (size_t)(tend - s.term_begin);
-                if (P.association == 0)
-                    P.s2.segs.push_back(SliceSeg{add_slice_block(P.ss, O.rows[o], s.K, 1, s.lda, tt, nt), slice_z(other)});
-                else
-                    P.s2.segs.push_back(SliceSeg{slice_x(other), add_slice_block(P.ss, O.cols[o], s.K, 0, s.lda, tt, nt)});
+                if (P.association == 0) {
+                    const int32_t z = slice_z(other);
+                    P.s2.segs.push_back(SliceSeg{add_slice_block(P.ss, O.rows[o], s.K, 1, s.lda, tt, nt, P.sz.blocks[z].koff), z});
+                } else {
+                    const int32_t x = slice_x(other);
+                    P.s2.segs.push_back(SliceSeg{x, add_slice_block(P.ss, O.cols[o], s.K, 0, s.lda, tt, nt, P.sx.blocks[x].koff)});
+                }
                 p2.segs.push_back(s);   // its term count is not limited here
                 p2.segs.back().term_count = (int32_t)nt;
                 j = jj;
