@@ -312,10 +312,12 @@ struct SplitTiling {
 // The exponents along K of a slice operand's blocks (koff, ks), from their data: make_plan asks for
 // those of the operand that meets Y
 using SliceColumns = std::function<std::vector<int32_t>(const SliceOperand&, bool z)>;
-// FP64 plan: two phases, the second sums first-stage products on the fly; once: applied a single
-// time, so that the slices of X and Z are made for it alone
+// FP64 plan: two phases, the second sums first-stage products on the fly.  By FMAs alone (fma), or
+// by slices where the rule of slice_engine takes them; once: applied a single time, so that
+// the slices of X and Z are made for it alone
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z,
-               const DevLayout& O, bool transX, bool transZ, bool once = false, const SliceColumns& columns = nullptr);
+               const DevLayout& O, bool transX, bool transZ, bool once = false, const SliceColumns& columns = nullptr,
+               bool fma = false);
 // Split-precision plan for the tcgen05 engine: op(X), Y and the chain-scaled
 // copies c*op(Z) in panels; phase 1 computes the intermediates T = op(X)Y into
 // panels, phase 2 the outputs as K-concatenations over chains.
@@ -336,7 +338,11 @@ PhasePlan make_product_plan(const DevLayout& A, const DevLayout& B, const DevLay
 // longest-first to the least-loaded CTA and stored CTA by CTA.
 void schedule_tma(PhasePlan& ph, int ncta, const std::vector<OpBlock>& A, const std::vector<OpBlock>& B,
                   int kstep = kUmmaBK);
-// The same for the FP64 slice engine, and its invariants (throws std::logic_error)
+// The same for the FP64 slice engine (throws SliceLimit where a phase needs more TMA descriptors than
+// fit the kernel parameter: the plan then runs by FMAs), and its invariants (throws std::logic_error)
+struct SliceLimit : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
 void schedule_slices(SlicePhase& ph, int ncta, const SliceOperand& A, const SliceOperand& B);
 void validate_slices(const SlicePhase& ph, const SliceOperand& A, const SliceOperand& B);
 // TMA box heights, the smallest that covers the tile: fine = the tile's rows

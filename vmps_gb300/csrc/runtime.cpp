@@ -1048,6 +1048,20 @@ static void ensure_io(vmps_pivot* p) {
 static void make_chunks(vmps_pivot* p, DevPlan& dp);
 static SplitTiling pivot_tiling(vmps_pivot* p);
 
+// An FP64 plan; one whose slices need more descriptors or memory than there are runs by FMAs
+template <typename Build>
+static void build_fp64(const vmps_ctx* c, DevPlan& dp, Build&& build) {
+    try {
+        build(false);
+        return;
+    } catch (const SliceLimit&) {
+    } catch (const std::bad_alloc&) {
+    }
+    if (c->device >= 0) cudaStreamSynchronize(c->stream);   // the lists of the dropped plan may still be read
+    dp = DevPlan();
+    build(true);
+}
+
 static DevPlan& get_plan(vmps_pivot* p, int prec) {
     if (prec != VMPS_PREC_FP64 && prec != VMPS_PREC_BF16X3 && prec != VMPS_PREC_TF32X3)
         throw std::invalid_argument("unknown precision");
@@ -1059,8 +1073,11 @@ static DevPlan& get_plan(vmps_pivot* p, int prec) {
             columns = [&](const SliceOperand& F, bool z) {
                 return slice_columns(F, (z ? p->dR : p->dL).as<double>(), p->st());
             };
-        dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, false, columns);
-        schedule_and_validate(dp.plan, p->ctx->num_sms);
+        build_fp64(p->ctx, dp, [&](bool fma) {
+            dp.plan = make_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, false, columns, fma);
+            schedule_and_validate(dp.plan, p->ctx->num_sms);
+            if (p->ctx->device >= 0) plan_to_device(dp, p->Vd, p->st());
+        });
     } else if (prec == VMPS_PREC_TF32X3) {
         dp.plan = make_split_plan(p->cs, p->Ld, p->Vd, p->Rd, p->Vd, false, false, 1, SplitTiling(), true);
         schedule_and_validate(dp.plan, p->ctx->num_sms);
@@ -1069,7 +1086,7 @@ static DevPlan& get_plan(vmps_pivot* p, int prec) {
         schedule_and_validate(dp.plan, p->ctx->num_sms);
     }
     if (p->ctx->device < 0) { dp.ready = true; return dp; }   // host-only: plan without device copies
-    plan_to_device(dp, p->Vd, p->st());
+    if (prec != VMPS_PREC_FP64) plan_to_device(dp, p->Vd, p->st());
     split_prepare(dp, p->dL.as<double>(), p->dR.as<double>(), p->st());
     if (prec == VMPS_PREC_BF16X3 && dp.plan.splitk == 1) make_chunks(p, dp);
     CK(cudaStreamSynchronize(p->st()));
@@ -2985,11 +3002,15 @@ static DevPlan& env_plan(vmps_env* e, int prec) {
     // left: X = Abra^dagger, Y = Eold, Z = Aket;  right: X = Aket, Y = Eold, Z = Abra^dagger
     const DevLayout& X = L ? e->Bd : e->Kd;
     const DevLayout& Z = L ? e->Kd : e->Bd;
-    if (prec == VMPS_PREC_FP64) dp.plan = make_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L, true);
-    else dp.plan = make_split_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
-    schedule_and_validate(dp.plan, e->ctx->num_sms);
+    auto build = [&](bool fma) {
+        if (prec == VMPS_PREC_FP64) dp.plan = make_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L, true, nullptr, fma);
+        else dp.plan = make_split_plan(e->cs, X, e->Ed, Z, e->Nd, L, !L);
+        schedule_and_validate(dp.plan, e->ctx->num_sms);
+        if (e->ctx->device >= 0) plan_to_device(dp, e->Ed, e->st());
+    };
+    if (prec == VMPS_PREC_FP64) build_fp64(e->ctx, dp, build);
+    else build(false);
     if (e->ctx->device < 0) { dp.ready = true; return dp; }
-    plan_to_device(dp, e->Ed, e->st());
     CK(cudaStreamSynchronize(e->st()));
     dp.ready = true;
     return dp;

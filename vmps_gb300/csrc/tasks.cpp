@@ -1314,6 +1314,9 @@ void schedule_slices(SlicePhase& ph, int ncta, const SliceOperand& A, const Slic
         }
         ph.cta_tiles[b + 1] = (int32_t)tiles.size();
     }
+    if ((int)ph.amaps.size() > kMaxMapsA || (int)ph.bmaps.size() > kMaxMapsB)
+        throw SliceLimit("slice plan: " + std::to_string(ph.amaps.size()) + " + " + std::to_string(ph.bmaps.size()) +
+                         " TMA descriptors in a phase");
     // sums over several segments: each flush by itself where few of them would be joined
     if (!ph.one_sum) ph.one_flush = (int64_t)ph.groups.size() * 3 <= ends * 4;
     ph.tiles.swap(tiles);
@@ -1380,7 +1383,7 @@ void validate_slices(const SlicePhase& ph, const SliceOperand& A, const SliceOpe
 }
 
 Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const DevLayout& Z, const DevLayout& O,
-               bool transX, bool transZ, bool once, const SliceColumns& columns) {
+               bool transX, bool transZ, bool once, const SliceColumns& columns, bool fma) {
     Plan P;
     // shapes: op(X) m x k, Y k x n, op(Z) n x p, out m x p
     auto xm = [&](int64_t x) { return transX ? X.cols[x] : X.rows[x]; };
@@ -1474,7 +1477,7 @@ Plan make_plan(const ChainSet& cs, const DevLayout& X, const DevLayout& Y, const
         };
         for (size_t j = 0; j < ipairs.size(); ++j) count(trows[j], tcols[j]);
         for (size_t o = 0; o < O.rows.size(); ++o) count(O.rows[o], O.cols[o]);
-        P.slices = slice_engine(std::min(f_xy, f_yz), tiles, once);
+        P.slices = !fma && slice_engine(std::min(f_xy, f_yz), tiles, once);
     }
 
     // ---- phase 1: T = op(X)*Y  (association 0)  or  U = Y*op(Z)  (association 1)
