@@ -911,10 +911,11 @@ static void run_plan(const DevPlan& dp, const Operands& ops, cudaStream_t st) {
 // Single-vector plans applied to nrhs vectors (ops.Y and ops.O: the first, the others vstride
 // elements apart).  An FP64 FMA plan takes as many in a launch as `T` holds first-stage buffers
 // for: at D = 256 a launch of one vector of the two-site Hubbard pivot runs 13 us for 2.6 MFLOP.
+constexpr int64_t kRhsLaunch = 65535;   // of the grid's second dimension
 static void run_plan_rhs(const DevPlan& dp, Operands ops, int nrhs, int64_t vstride, const DBuf& T, cudaStream_t st) {
     const int64_t tbytes = std::max<int64_t>(dp.plan.T.total, 1) * 8;
     const bool fma = !dp.plan.split && !dp.plan.slices;
-    const int batch = fma && T.p ? (int)std::min<int64_t>(nrhs, std::max<int64_t>(1, (int64_t)T.bytes / tbytes)) : 1;
+    const int batch = fma && T.p ? (int)std::min({(int64_t)nrhs, kRhsLaunch, std::max<int64_t>(1, (int64_t)T.bytes / tbytes)}) : 1;
     const double* Y = ops.Y;
     double* O = ops.O;
     const PenaltyArgs* pen = ops.pen;
@@ -939,7 +940,7 @@ static void run_plan_rhs(const DevPlan& dp, Operands ops, int nrhs, int64_t vstr
 constexpr int64_t kRhsBytes = int64_t(512) << 20;
 static void alloc_rhs(DBuf& T, const DevPlan& dp, int nrhs, cudaStream_t st) {
     const int64_t tbytes = std::max<int64_t>(dp.plan.T.total, 1) * 8;
-    const int64_t m = std::min<int64_t>(nrhs, kRhsBytes / tbytes);
+    const int64_t m = std::min({(int64_t)nrhs, kRhsLaunch, kRhsBytes / tbytes});
     if (dp.plan.split || dp.plan.slices || m < 2) return;
     try {
         T.alloc((size_t)(m * tbytes), st, false);
