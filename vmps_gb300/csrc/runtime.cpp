@@ -81,11 +81,23 @@ struct DevPool {
     cudaMemPool_t pool = nullptr;
     int contexts = 0;
 };
-// a context's stream as its buffers know it: they may outlive the context
+// a context's stream as its buffers know it: they may outlive the context, and go on another thread
+// than the one that works with it
 struct StreamRef {
     std::mutex mu;
     cudaStream_t st = nullptr;     // null once the context is gone (its work has finished then)
     cudaMemPool_t pool = nullptr;
+    bool capturing = false;        // a free would become part of the graph, and run whenever that does:
+    std::vector<void*> held;       // buffers released meanwhile
+    // (mu is held)
+    void free(void* p) noexcept {
+        if (!st) cudaFree(p);
+        else if (!capturing) cudaFreeAsync(p, st);
+        else try {
+            held.push_back(p);
+        } catch (const std::bad_alloc&) {   // no host memory left for the list: the buffer stays
+        }
+    }
 };
 static std::mutex g_pool_mu;
 static std::map<int, DevPool> g_pools;                                   // by device
@@ -132,6 +144,47 @@ static void unregister_stream(int device, cudaStream_t st) {
     if (--dp.contexts == 0) cudaMemPoolTrimTo(dp.pool, 0);
 }
 
+// A capture of a context's stream; without an end it is dropped.  Buffers released meanwhile, on whatever
+// thread, are freed at its end.
+class StreamCapture {
+  public:
+    explicit StreamCapture(cudaStream_t st) : st_(st), ref_(stream_ref(st)) {
+        std::unique_lock<std::mutex> lock;
+        if (ref_) lock = std::unique_lock<std::mutex>(ref_->mu);
+        CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
+        open_ = true;
+        if (ref_) ref_->capturing = true;
+    }
+    StreamCapture(const StreamCapture&) = delete;
+    StreamCapture& operator=(const StreamCapture&) = delete;
+    ~StreamCapture() {
+        cudaGraph_t g = nullptr;
+        if (open_ && close(&g) == cudaSuccess && g) cudaGraphDestroy(g);
+    }
+    cudaGraph_t end() {
+        cudaGraph_t g = nullptr;
+        CK(close(&g));
+        return g;
+    }
+
+  private:
+    cudaError_t close(cudaGraph_t* g) noexcept {
+        open_ = false;
+        std::unique_lock<std::mutex> lock;
+        if (ref_) lock = std::unique_lock<std::mutex>(ref_->mu);
+        const cudaError_t e = cudaStreamEndCapture(st_, g);
+        if (ref_) {
+            ref_->capturing = false;
+            for (void* p : ref_->held) ref_->free(p);
+            ref_->held.clear();
+        }
+        return e;
+    }
+    cudaStream_t st_;
+    std::shared_ptr<StreamRef> ref_;
+    bool open_ = false;
+};
+
 struct DBuf {
     void* p = nullptr;
     size_t bytes = 0;
@@ -154,8 +207,7 @@ struct DBuf {
         if (!p) return;
         if (ref) {
             std::lock_guard<std::mutex> lock(ref->mu);
-            if (ref->st) cudaFreeAsync(p, ref->st);
-            else cudaFree(p);
+            ref->free(p);
         } else {
             cudaFree(p);
         }
@@ -1840,8 +1892,9 @@ int vmps_pivot_set_penalty(vmps_pivot* p, int nproj, const double* A0, double Ep
 }
 
 // Destroy functions never touch the owning context or pivot: callers (and
-// garbage collectors) may release objects in any order.  cudaFree waits for
-// the device work that still uses the memory.
+// garbage collectors) may release objects in any order and on any thread.  Buffers
+// are freed in the order of the context's stream, after the work that still uses them;
+// those released while that stream is captured, at the capture's end.
 int vmps_pivot_destroy(vmps_pivot* p) {
     delete p;
     return VMPS_OK;
@@ -2029,10 +2082,9 @@ int vmps_hxv_time(vmps_pivot* p, const vmps_dvec* vin, vmps_dvec* vout, int prec
     if (use_graph) {
         if (!p->graph[prec] || p->graph_in[prec] != vi || p->graph_out[prec] != vo) {
             if (p->graph[prec]) { cudaGraphExecDestroy(p->graph[prec]); p->graph[prec] = nullptr; }
-            cudaGraph_t g;
-            CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            StreamCapture cap(st);
             run_plan(dp, ops, st);
-            CK(cudaStreamEndCapture(st, &g));
+            cudaGraph_t g = cap.end();
             cudaGraphExec_t ge;
             CK(cudaGraphInstantiate(&ge, g, 0));
             cudaGraphDestroy(g);
@@ -2294,15 +2346,12 @@ LzResult lz_run(vmps_pivot* p, LzWork& W, int prec, int kmax, double tol_eigval,
     }
     // one iteration = the HxV plan + the four step kernels, captured once
     cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    try {
+    {
+        StreamCapture cap(st);
         run_plan(dp, ops, st);
         CK(launch_lz_step(a, W.sh.per_thread, st));
-    } catch (...) {
-        if (cudaStreamEndCapture(st, &g) == cudaSuccess && g) cudaGraphDestroy(g);
-        throw;
+        g = cap.end();
     }
-    CK(cudaStreamEndCapture(st, &g));
     cudaGraphExec_t ge = nullptr;
     const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
@@ -2789,24 +2838,13 @@ static int chebyshev_moments(vmps_pivot* p, const double* v0, int nrhs, int nmom
         c.nparts = nparts;
         for (int j = 0; j <= nparts; ++j) c.pbeg[j] = pbeg[j];
         Operands ops = pivot_ops(p);
-        cudaGraph_t gr = nullptr;
-        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-        try {
-            if (prec == VMPS_PREC_BF16X3) {
-                ops.Y = c.tn;
-                ops.O = Wb.as<double>();
-                run_plan(dp, ops, st);
-            } else {
-                ops.Y = c.tn;
-                ops.O = Wb.as<double>();
-                run_plan_rhs(dp, ops, nrhs, n, T, st);
-            }
-            CK(launch_cheb_step(c, sh.per_thread, st));
-        } catch (...) {
-            if (cudaStreamEndCapture(st, &gr) == cudaSuccess && gr) cudaGraphDestroy(gr);
-            throw;
-        }
-        CK(cudaStreamEndCapture(st, &gr));
+        ops.Y = c.tn;
+        ops.O = Wb.as<double>();
+        StreamCapture cap(st);
+        if (prec == VMPS_PREC_BF16X3) run_plan(dp, ops, st);
+        else run_plan_rhs(dp, ops, nrhs, n, T, st);
+        CK(launch_cheb_step(c, sh.per_thread, st));
+        cudaGraph_t gr = cap.end();
         const cudaError_t ie = cudaGraphInstantiate(&g[r], gr, 0);
         cudaGraphDestroy(gr);
         CK(ie);
