@@ -1292,6 +1292,17 @@ static void hxv_host_pipelined(vmps_pivot* p, DevPlan& dp, const double* vin, do
     ops.err = p->ctx->err;
     ops.wait_budget = p->ctx->wait_budget;
     const int kin = (int)ch.in.size(), kout = (int)ch.out.size();
+    // an error on the way waits for the copies in flight: the caller's vectors and the buffers, whose
+    // release follows the compute stream alone, must outlast them
+    struct Drain {
+        cudaStream_t copies, work;
+        bool done = false;
+        ~Drain() {
+            if (done) return;
+            cudaStreamSynchronize(copies);
+            cudaStreamSynchronize(work);
+        }
+    } drain{xs, cs};
     // the copy stream starts after everything already queued on the compute stream
     CK(cudaEventRecord(ch.ev_start, cs));
     CK(cudaStreamWaitEvent(xs, ch.ev_start, 0));
@@ -1320,6 +1331,7 @@ static void hxv_host_pipelined(vmps_pivot* p, DevPlan& dp, const double* vin, do
     }
     CK(cudaStreamSynchronize(xs));
     CK(cudaStreamSynchronize(cs));
+    drain.done = true;
 }
 
 static void require_device(const vmps_ctx* c) {
