@@ -35,8 +35,9 @@ namespace vmps {
 // tensors are 5 to 200 wide.  64 x 64 DMMA tiles left an 11 x 11 block to one
 // warp of one SM (72 us per launch at D = 64, now ~11); here the elements of a
 // tile spread over all four quadrants without rounding, and the tiles over more
-// SMs.  Large blocks gain as well: whole D = 1024 and 4096 two-site HxVs went from
-// 0.76 to 0.43 ms and from 17.9 to 16.3 ms, the FP64 pipe bounding both.  Small
+// SMs.  Large blocks gain as well: by this kernel, whole D = 1024 and 4096 two-site HxVs went from
+// 0.76 to 0.43 ms and from 17.9 to 16.3 ms, the FP64 pipe bounding both (by slices, which plans of
+// that size take unless pinned, they run 0.20 and 2.1 ms).  Small
 // ones are bound by the latency of the segment chain, so the segments and terms
 // of a tile come to shared memory first and each K chunk's loads are issued one
 // chunk ahead.  Several right-hand sides share a launch (blockIdx.y): one launch

@@ -526,7 +526,7 @@ static void encode_panel_map(CUtensorMap* m, const PanelArena& ar, const DBuf& a
 }
 
 // A slice panel class as a 3-d tensor: 32 elements, its rows, its (K step, slice) pairs;
-// boxes of one K step's eight slices of the key's rows, 64-byte swizzle
+// boxes of one K step's seven slices of the key's rows, 64-byte swizzle
 static void encode_slice_map(CUtensorMap* m, const PanelArena& ar, const DBuf& arena, const MapKey& k) {
     const PanelClass& c = ar.cls.at(k.cls);
     if (k.rows < 16 || k.rows > 256 || k.rows % 16 != 0) throw std::logic_error("TMA box rows out of range");

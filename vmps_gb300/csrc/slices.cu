@@ -333,7 +333,8 @@ __device__ __forceinline__ int slice_cvt(uint32_t v) {
 }
 
 // A flushed element, the orders S_0..S_6 (FP32, exact integers) summed in units of 2^-49 of
-// S_0's: hi 256 + lo, |hi| < 2^61
+// S_0's: hi 256 + lo, |hi| < 1.1 2^61 and |lo| < 2^29, so that the sums of three fit 64
+// and 32 bits
 struct SliceSum { int64_t hi; int lo; };
 // Integers come from adding 1.5 * 2^23, which holds |S| <= 2^22: S_0 and S_1 always (<= 2^20,
 // 2^22), S_2 .. S_6 (<= 2^25) in all but contrived sums, for which `off` becomes nonzero
@@ -361,13 +362,14 @@ __device__ __forceinline__ SliceSum slice_sum_any(const uint32_t (&v)[kSlices][N
                 (int64_t)s[4] * (1 << 5), s[5] * 16 + ((s[6] + 16) >> 5)};
 }
 
-// x in units of 2^(e - 63), as 64 bits in units of 2^(e - 63) or, from 2^61 on, 2^(e - 55)
+// x, one flush or a sum of up to three, in units of 2^(e - 63), as 64 bits in units of 2^(e - 63) or, from
+// |hi| = 2^53 on, 2^(e - 55): |result| < 2^61 + 2^31 or < 3.4 2^61
 __device__ __forceinline__ int64_t slice_pack(const SliceSum& x, int& e) {
     const bool big = (((uint32_t)(x.hi >> 32) + 0x200000u) & 0xFFC00000u) != 0;   // |hi| >= 2^53
     e -= big ? 55 : 63;
     return big ? x.hi + ((x.lo + 128) >> 8) : x.hi * 256 + x.lo;
 }
-// x 2^e, rounded to nearest, by integer operations; |e| < 1000 and |x| >= 2^36 (else `small`
+// x 2^e, rounded to nearest, by integer operations; |e| < 1000 and 2^36 <= |x| < 2^63 (below, `small`
 // becomes nonzero)
 __device__ __forceinline__ double slice_to_double(int64_t x, int e, uint32_t& small) {
     const uint32_t s = (uint32_t)(x >> 63);

@@ -1186,7 +1186,7 @@ void add_slice_tiles(SlicePhase& ph, int64_t c_off, int64_t ldc, int64_t m, int6
             ph.tile_segs.push_back({sb, se});
         }
 }
-// TMA box heights of A: the tile's rows rounded up to 16, or (fewer descriptors) 16, 32, 64 or 112
+// TMA box heights of A: the tile's rows rounded up to 16, or (fewer descriptors) 16, 32, 64 or 128
 int32_t slice_box_a(int32_t tm, bool fine) {
     return std::min<int32_t>(kSliceTileM, fine ? std::max<int32_t>(16, (tm + 15) / 16 * 16) : box_rows_a(tm, false));
 }
