@@ -2528,7 +2528,7 @@ constexpr double kRoundMinRatio = 10;
 
 // The ratio comes from a cost model of the plans (not from timings, so that the
 // choice, and with it every result bit, does not depend on the run): GEMM work at
-// fixed rates (FP64 0.87 TFLOP/s, bf16 tensor work as issued 530 TFLOP/s; the exact
+// fixed rates (FP64 0.87 TFLOP/s, bf16 tensor work as issued 530 TFLOP/s; the
 // slices of large FP64 plans run faster, but a changed rate would change which
 // solves refine by rounds, and with it their results), the Lanczos step's vector reads and writes at 5 TB/s,
 // and 3 us per launch.
